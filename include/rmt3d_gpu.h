@@ -367,11 +367,15 @@ int rmt3d_div_u_noalloc(const int sys_size[3], const int periodic[3], const doub
  * running every colour pass there.  Both give the same bits. */
 int rmt3d_scene_set_smoother(rmt3d_scene *s, int mode);
 
-/* The coarse part of every V-cycle -- the levels of at most `pts` points
- * below the finest, down to the coarsest, with their smoothing, residuals,
- * transfers and the dense coarsest solve -- as one launch of a thread-block
- * cluster (16 CTAs, or 8) instead of one full-GPU launch per phase; 0 keeps
- * per-phase launches.  No counterpart in the reference. */
+/* The part of every V-cycle on the levels of at most `pts` points, down to the
+ * coarsest, with their smoothing, residuals, transfers and the dense coarsest
+ * solve, as one launch of a thread-block cluster (16 CTAs, or 8) that holds
+ * those levels in shared memory, instead of one full-GPU launch per phase
+ * (the same bits).  Levels too large for the cluster's shared memory keep
+ * per-phase launches; 0 keeps them for every level.  A new scene hands over
+ * as many levels as fit, until this call, rmt3d_scene_set_smoother or a
+ * one-block coarse sub-cycle (rmt3d_scene_set_schedule) chooses otherwise.
+ * No counterpart in the reference. */
 int rmt3d_scene_set_coarse_cluster(rmt3d_scene *s, int pts);
 
 /* Block shape of the bulk stencil kernels of the step (stress, edge states,

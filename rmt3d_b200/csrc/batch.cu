@@ -270,8 +270,8 @@ extern "C" int rmt3d_batch_autotune(rmt3d_batch *b, int probe_steps, int *tuned_
     drop_groups(b);
     static const int smooth[][2] = {{2, 2}, {1, 1}, {1, 2}, {2, 1}, {3, 3}};
     // (whole solve as one cluster launch, smoother: 0 colour passes, 1 tiled
-    // sweeps, largest level of the coarse part run as one cluster launch)
-    static const int launch[][3] = {{1, 0, 0}, {0, 0, 0}, {0, 1, 0}, {0, 0, 5000}, {0, 0, 40000}, {0, 1, 5000}};
+    // sweeps, largest level of the part run as one cluster launch)
+    static const int launch[][3] = {{1, 0, 0}, {0, 0, 40000}, {0, 0, 5000}, {0, 0, 0}, {0, 1, 0}};
     std::map<std::array<int, 8>, int> first;
     for (size_t i = 0; i < b->descs.size(); i++)
         if (!first.count(tune_key(b->descs[i]))) first[tune_key(b->descs[i])] = (int)i;
@@ -300,8 +300,8 @@ extern "C" int rmt3d_batch_autotune(rmt3d_batch *b, int probe_steps, int *tuned_
                 for (size_t q = 0; q < cs.size(); q++) {
                     cand &c = cs[round % 2 ? cs.size() - 1 - q : q];
                     if (!c.ok) continue;
-                    if (rmt3d_scene_set_mg_launch(probe, c.cl) || rmt3d_scene_set_coarse_cluster(probe, c.cc) ||
-                        rmt3d_scene_set_schedule(probe, c.vd, c.vu, 0) || rmt3d_scene_set_smoother(probe, c.sm) ||
+                    if (rmt3d_scene_set_mg_launch(probe, c.cl) || rmt3d_scene_set_schedule(probe, c.vd, c.vu, 0) ||
+                        rmt3d_scene_set_smoother(probe, c.sm) || rmt3d_scene_set_coarse_cluster(probe, c.cc) ||
                         rmt3d_scene_set_block_shape(probe, c.bs)) {
                         c.ok = false;  // e.g. clusters unavailable on this device
                         continue;

@@ -350,6 +350,7 @@ int mg_solver::build_dense(cudaStream_t st) {
 int mg_solver::set_coarse(int pts) {
     coarse_pts = vd ? 0 : pts;
     pts = coarse_pts;
+    if (pts > 0 && cluster_coarse_pts == kSlabAuto) set_cluster_coarse(0);
     invalidate();
     cf = (int)lv.size() - 1;
     for (int l = 0; l < (int)lv.size(); l++)
@@ -481,6 +482,8 @@ int mg_solver::setup(mg_kind k, const int n[3], const int prd[3], bool mixed_for
     if (tile_setup()) return fail(RMT3D_ERR_CUDA, "tiled sweep kernel configuration failed");
 
     setup_cluster();
+    slab_csize = slab_cluster_size();
+    set_cluster_coarse(cluster_coarse_pts);
     {
         const char *e = getenv("RMT3D_MG_CLUSTER");
         if (e && e[0] == '1') use_cluster = true;
@@ -590,12 +593,14 @@ static pmg_args coarse_args(const mg_solver &m) {
     return A;
 }
 
+// The first level of at most `pts` points whose part of the V-cycle fits a
+// cluster's shared memory.  kSlabAuto takes the largest part that fits.
 int mg_solver::set_cluster_coarse(int pts) {
     cluster_coarse_pts = pts;
     ccl = -1;
-    if (pts > 0 && cluster_size > 0)
-        for (int l = 1; l + 1 < (int)lv.size(); l++)
-            if (lv[l].npts() <= (size_t)pts) {
+    if (pts != 0 && slab_csize > 0 && dense)
+        for (int l = 0; l + 1 < (int)lv.size(); l++)
+            if ((pts == kSlabAuto || lv[l].npts() <= (size_t)pts) && slab_fits(*this, l)) {
                 ccl = l;
                 break;
             }
@@ -606,8 +611,8 @@ int mg_solver::set_cluster_coarse(int pts) {
 int mg_solver::cycle(int l, cudaStream_t st) {
     mg_level &F = lv[l];
     lvl_dev fd = dev_of(F);
-    if (l == ccl) {
-        LAUNCH(coarse_cluster(*this, l, false, st));
+    if (slab_at(l)) {
+        LAUNCH(slab_cycle_launch(*this, l, false, st));
         return 0;
     }
     if (l == cf && l < (int)lv.size() - 1) {
@@ -644,8 +649,8 @@ int mg_solver::cycle(int l, cudaStream_t st) {
 int mg_solver::cycle_f32(int l, cudaStream_t st) {
     mg_level &F = lv[l];
     lvl_dev fd = dev_of(F);
-    if (l == ccl) {
-        LAUNCH(coarse_cluster(*this, l, true, st));
+    if (slab_at(l)) {
+        LAUNCH(slab_cycle_launch(*this, l, true, st));
         return 0;
     }
     if (l == cf && l < (int)lv.size() - 1) {

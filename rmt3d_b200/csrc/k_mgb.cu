@@ -223,12 +223,12 @@ int mg_group::setup(const std::vector<mg_solver *> &solvers, cudaStream_t st) {
     v_up = s0.v_up;
     smoother = s0.smoother;
     ccl = s0.ccl;
-    csize = s0.cluster_size;
+    csize = s0.slab_csize;
     dense = s0.dense;
     for (const mg_solver *m : solvers) {
         bool same = m->kind == kind && m->lv.size() == lv.size() && m->mixed == mixed && m->exact == exact &&
                     m->vd == vd && m->rtol == rtol && m->dense == dense && m->v_down == v_down && m->v_up == v_up &&
-                    m->smoother == smoother && m->ccl == ccl && m->cluster_size == csize;
+                    m->smoother == smoother && m->ccl == ccl && m->slab_csize == csize;
         for (size_t l = 0; same && l < lv.size(); l++)
             for (int d = 0; d < 3; d++) same = same && m->lv[l].n[d] == lv[l].n[d] && m->lv[l].prd[d] == lv[l].prd[d];
         if (!same) return fail(RMT3D_ERR_INVALID, "scenes of a multigrid group must match in size, form and schedule");
@@ -353,7 +353,7 @@ static int cycle_b(mg_group &g, int l, cudaStream_t st) {
     const mg_level &F = g.lv[l];
     const int nl = (int)g.lv.size();
     if (l == g.ccl) {
-        coarse_cluster_b(g.dargs, g.run, g.B, l, g.csize, sizeof(T) == 4, st);
+        slab_cycle_launch_b(g, l, sizeof(T) == 4, st);
         g.body_kernels++;
         return 0;
     }

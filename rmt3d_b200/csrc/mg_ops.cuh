@@ -338,6 +338,32 @@ struct pmg_args {
     int v_up, v_down;
 };
 
+// the columns (or rows) of one parity: their number, the number off the rim
+// of the plane, whether the first one lies on the rim
+struct slab_col {
+    int n, in, lo;
+    unsigned inv_in;
+};
+// One level of a V-cycle part held in shared memory, cut into slabs of q
+// planes (k_mgs.cu).  Offsets and strides in elements of a CTA's arrays.
+struct slab_level {
+    int n0, n1, n2, p0, p1, p2;
+    int q;              // planes per CTA
+    int H, RS, PX, PR;  // half row, row, plane of x (with ghosts), plane of r
+    int ox, orr, os, oi;  // x, r, residual, 1/rho
+    // reciprocals for index division
+    unsigned inv_n0, inv_n1, inv_q, inv_w0, inv_w1, inv_half, inv_in[4], inv_rim[4];
+    slab_col cx[2], cy[2];  // FEM: the colours' columns and rows
+};
+struct slab_args {
+    int l0, nlev, csize, load_x;
+    int zero_elems;  // x and 1/rho arrays, zeroed at the start
+    int dense_off;   // bytes: the coarsest right-hand side in FP64
+    int bar_off;     // bytes: two mbarriers and a flag
+    int pass_off;    // bytes: the passes' tables
+    slab_level lv[kMaxLev];
+};
+
 __device__ __forceinline__ lvl_dev ldev(const pmg_level &L) {
     return lvl_dev{L.n[0], L.n[1], L.n[2], L.prd[0], L.prd[1], L.prd[2]};
 }

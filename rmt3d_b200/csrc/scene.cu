@@ -2875,7 +2875,7 @@ void scene_schedule(rmt3d_scene *s, int out[5]) {
 extern "C" int rmt3d_scene_set_coarse_cluster(rmt3d_scene *s, int pts) {
     if (!s) return fail(RMT3D_ERR_INVALID, "null scene");
     if (pts < 0) return fail(RMT3D_ERR_INVALID, "negative level size");
-    if (pts > 0 && (!s->mac.cluster_size || !s->fem.cluster_size))
+    if (pts > 0 && (!s->mac.slab_csize || !s->fem.slab_csize))
         return fail(RMT3D_ERR_UNSUPPORTED, "thread-block clusters of 8 or more CTAs are not available");
     s->mac.set_cluster_coarse(pts);
     s->fem.set_cluster_coarse(pts);
@@ -2894,9 +2894,13 @@ extern "C" int rmt3d_scene_set_block_shape(rmt3d_scene *s, int shape) {
 extern "C" int rmt3d_scene_set_smoother(rmt3d_scene *s, int mode) {
     if (!s) return fail(RMT3D_ERR_INVALID, "null scene");
     if (mode < 0 || mode > 1) return fail(RMT3D_ERR_INVALID, "smoother mode must be 0 (colour passes) or 1 (tiled sweeps)");
-    s->mac.smoother = s->fem.smoother = mode;
-    s->mac.invalidate();
-    s->fem.invalidate();
+    // a smoother named by the caller runs on every level: no cluster launch
+    // unless rmt3d_scene_set_coarse_cluster asks for one
+    for (mg_solver *m : {&s->mac, &s->fem}) {
+        m->smoother = mode;
+        if (m->cluster_coarse_pts == kSlabAuto) m->set_cluster_coarse(0);
+        m->invalidate();
+    }
     mark_dirty(s);
     return RMT3D_OK;
 }
