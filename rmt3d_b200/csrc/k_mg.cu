@@ -39,26 +39,27 @@ namespace rmt3d {
 
 // ---- single-scene phase kernels (bodies in mg_body.cuh) ---------------------
 template <typename T>
-__global__ void k_mac_rb(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour, const T *__restrict__ ri) {
-    body_mac_rb<T>(L, x, r, colour, ri, blockIdx.x, blockIdx.y, blockIdx.z);
+__global__ void __launch_bounds__(256) k_mac_rb(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour,
+                                                const T *__restrict__ ri, unsigned inv) {
+    body_mac_rb<T>(L, x, r, colour, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
 template <typename T>
-__global__ void k_fem_gs(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour, const T *__restrict__ ri) {
-    body_fem_gs<T>(L, x, r, colour, ri, blockIdx.x, blockIdx.y, blockIdx.z);
+__global__ void __launch_bounds__(256) k_fem_gs(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour,
+                                                const T *__restrict__ ri, unsigned inv) {
+    body_fem_gs<T>(L, x, r, colour, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
 template <typename T, int KIND>
-__global__ void k_resid(lvl_dev L, const T *__restrict__ x, const T *__restrict__ r, T *__restrict__ res,
-                        unsigned long long *mx, const T *__restrict__ ri) {
-    const double a = body_resid<T, KIND>(L, x, r, res, ri, blockIdx.x, blockIdx.y, blockIdx.z);
-    if (mx) warp_max_into(a, mx);
+__global__ void __launch_bounds__(256) k_resid(lvl_dev L, const T *__restrict__ x, const T *__restrict__ r,
+                                               T *__restrict__ res, const T *__restrict__ ri, unsigned inv) {
+    body_resid<T, KIND>(L, x, r, res, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
 // the control's max-norm residual, computed only when the control will read it
 template <int KIND>
-__global__ void k_resid_ctl(lvl_dev L, const double *__restrict__ x, const double *__restrict__ r,
-                            unsigned long long *mx, const double *__restrict__ ri, const mg_ctl *c) {
+__global__ void __launch_bounds__(256) k_resid_ctl(lvl_dev L, const double *__restrict__ x,
+                                                   const double *__restrict__ r, unsigned long long *mx,
+                                                   const double *__restrict__ ri, const mg_ctl *c, unsigned inv) {
     if (!c->need_res) return;
-    const double a = body_resid<double, KIND>(L, x, r, nullptr, ri, blockIdx.x, blockIdx.y, blockIdx.z);
-    warp_max_into(a, mx);
+    block_max_into(body_resid_max<KIND>(L, x, r, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y), mx);
 }
 template <typename T>
 __global__ void k_mac_restrict(lvl_dev F, lvl_dev C, const T *__restrict__ res, T *__restrict__ rc,
@@ -66,9 +67,10 @@ __global__ void k_mac_restrict(lvl_dev F, lvl_dev C, const T *__restrict__ res, 
     body_mac_restrict<T>(F, C, res, rc, xc0, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 template <int KIND>
-__global__ void k_resid_to_f32(lvl_dev L, const double *__restrict__ x, const double *__restrict__ r,
-                               const double *__restrict__ ri, float *__restrict__ rs, float *__restrict__ xs) {
-    body_resid_to_f32<KIND>(L, x, r, ri, rs, xs, blockIdx.x, blockIdx.y, blockIdx.z);
+__global__ void __launch_bounds__(256) k_resid_to_f32(lvl_dev L, const double *__restrict__ x,
+                                                      const double *__restrict__ r, const double *__restrict__ ri,
+                                                      float *__restrict__ rs, float *__restrict__ xs, unsigned inv) {
+    body_resid_to_f32<KIND>(L, x, r, ri, rs, xs, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
 template <typename T>
 __global__ void k_mac_prolong(lvl_dev F, lvl_dev C, T *__restrict__ x, const T *__restrict__ xc) {
@@ -172,6 +174,15 @@ static lvl_dev dev_of(const mg_level &l) { return lvl_dev{l.n[0], l.n[1], l.n[2]
 
 static dim3 blk3() { return dim3(32, 4, 2); }
 static dim3 grid3(int a, int b, int c) { return dim3((a + 31) / 32, (b + 3) / 4, (c + 1) / 2); }
+// one plane's line of points (mg_body.cuh) per block row: every point, or one
+// colour's
+static dim3 grid_line(const mg_level &L) { return dim3((L.n[0] * L.n[1] + 255) / 256, L.n[2]); }
+static dim3 grid_colour(mg_kind kind, const mg_level &L) {
+    const int rows = kind == MG_MAC ? L.n[1] : (L.n[1] + 1) / 2;
+    return dim3(((L.n[0] + 1) / 2 * rows + 255) / 256, L.n[2]);
+}
+// prolongation: a thread per fine column and coarse row pair
+static dim3 grid_prolong(const mg_level &F, const mg_level &C) { return grid3(F.n[0], C.n[1], C.n[2]); }
 
 template <typename T, int KIND, bool VD>
 static int tile_attr(const void *fn) {
@@ -517,17 +528,17 @@ int mg_solver::smooth(int l, int sweeps, int cur, cudaStream_t st) {
             if (timed) prof->end(st, npts, 8.0 * npts * (L.ri ? 4 : 3));
             cur ^= 1;
         } else if (kind == MG_MAC) {
-            dim3 g((L.n[0] / 2 + 1 + 31) / 32, (L.n[1] + 3) / 4, (L.n[2] + 1) / 2);
+            const dim3 g = grid_colour(kind, L);
             for (int c = 0; c < 2; c++) {
                 if (timed) prof->begin(st);
-                LAUNCH(k_mac_rb<double><<<g, blk3(), 0, st>>>(d, xb[cur], L.r, c, L.ri));
+                LAUNCH(k_mac_rb<double><<<g, 256, 0, st>>>(d, xb[cur], L.r, c, L.ri, line_inv((L.n[0] + 1) / 2)));
                 if (timed) prof->end(st, npts / 2, 8.0 * (npts + npts / 2 + npts / 2));
             }
         } else {
-            dim3 g(((L.n[0] + 1) / 2 + 31) / 32, ((L.n[1] + 1) / 2 + 3) / 4, (L.n[2] + 1) / 2);
+            const dim3 g = grid_colour(kind, L);
             for (int c = 0; c < 4; c++) {
                 if (timed) prof->begin(st);
-                LAUNCH(k_fem_gs<double><<<g, blk3(), 0, st>>>(d, xb[cur], L.r, c, L.ri));
+                LAUNCH(k_fem_gs<double><<<g, 256, 0, st>>>(d, xb[cur], L.r, c, L.ri, line_inv((L.n[0] + 1) / 2)));
                 if (timed) prof->end(st, npts / 4, 8.0 * (npts + npts / 4 + npts / 4));
             }
         }
@@ -548,17 +559,17 @@ int mg_solver::smooth_f32(int l, int sweeps, int cur, cudaStream_t st) {
             if (timed) prof->end(st, npts, 4.0 * npts * (L.ris ? 4 : 3));
             cur ^= 1;
         } else if (kind == MG_MAC) {
-            dim3 g((L.n[0] / 2 + 1 + 31) / 32, (L.n[1] + 3) / 4, (L.n[2] + 1) / 2);
+            const dim3 g = grid_colour(kind, L);
             for (int c = 0; c < 2; c++) {
                 if (timed) prof->begin(st);
-                LAUNCH(k_mac_rb<float><<<g, blk3(), 0, st>>>(d, xb[cur], L.rs, c, L.ris));
+                LAUNCH(k_mac_rb<float><<<g, 256, 0, st>>>(d, xb[cur], L.rs, c, L.ris, line_inv((L.n[0] + 1) / 2)));
                 if (timed) prof->end(st, npts / 2, 4.0 * (npts + npts / 2 + npts / 2));
             }
         } else {
-            dim3 g(((L.n[0] + 1) / 2 + 31) / 32, ((L.n[1] + 1) / 2 + 3) / 4, (L.n[2] + 1) / 2);
+            const dim3 g = grid_colour(kind, L);
             for (int c = 0; c < 4; c++) {
                 if (timed) prof->begin(st);
-                LAUNCH(k_fem_gs<float><<<g, blk3(), 0, st>>>(d, xb[cur], L.rs, c, L.ris));
+                LAUNCH(k_fem_gs<float><<<g, 256, 0, st>>>(d, xb[cur], L.rs, c, L.ris, line_inv((L.n[0] + 1) / 2)));
                 if (timed) prof->end(st, npts / 4, 4.0 * (npts + npts / 4 + npts / 4));
             }
         }
@@ -631,18 +642,18 @@ int mg_solver::cycle(int l, cudaStream_t st) {
     double *xb[2] = {F.x, F.res};
     mg_level &C = lv[l + 1];
     lvl_dev cd = dev_of(C);
-    dim3 gf = grid3(F.n[0], F.n[1], F.n[2]), gc = grid3(C.n[0], C.n[1], C.n[2]);
+    const dim3 gc = grid3(C.n[0], C.n[1], C.n[2]);
     if (kind == MG_MAC) {
-        LAUNCH((k_resid<double, 0><<<gf, blk3(), 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], nullptr, F.ri)));
+        LAUNCH((k_resid<double, 0><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]))));
         LAUNCH(k_mac_restrict<double><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.r, C.x));
     } else {
-        LAUNCH((k_resid<double, 1><<<gf, blk3(), 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], nullptr, F.ri)));
+        LAUNCH((k_resid<double, 1><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]))));
         LAUNCH(k_fem_restrict<double><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.r, C.x));
     }
     const int cc = cycle(l + 1, st);
     const double *xc = cc ? C.res : C.x;
-    if (kind == MG_MAC) LAUNCH(k_mac_prolong<double><<<gf, blk3(), 0, st>>>(fd, cd, xb[cur], xc));
-    else LAUNCH(k_fem_prolong<double><<<gf, blk3(), 0, st>>>(fd, cd, xb[cur], xc));
+    if (kind == MG_MAC) LAUNCH(k_mac_prolong<double><<<grid_prolong(F, C), blk3(), 0, st>>>(fd, cd, xb[cur], xc));
+    else LAUNCH(k_fem_prolong<double><<<grid_prolong(F, C), blk3(), 0, st>>>(fd, cd, xb[cur], xc));
     return smooth(l, v_up, cur, st);
 }
 
@@ -667,18 +678,18 @@ int mg_solver::cycle_f32(int l, cudaStream_t st) {
     float *xb[2] = {F.xs, F.ress};
     mg_level &C = lv[l + 1];
     lvl_dev cd = dev_of(C);
-    dim3 gf = grid3(F.n[0], F.n[1], F.n[2]), gc = grid3(C.n[0], C.n[1], C.n[2]);
+    const dim3 gc = grid3(C.n[0], C.n[1], C.n[2]);
     if (kind == MG_MAC) {
-        LAUNCH((k_resid<float, 0><<<gf, blk3(), 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], nullptr, F.ris)));
+        LAUNCH((k_resid<float, 0><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]))));
         LAUNCH(k_mac_restrict<float><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.rs, C.xs));
     } else {
-        LAUNCH((k_resid<float, 1><<<gf, blk3(), 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], nullptr, F.ris)));
+        LAUNCH((k_resid<float, 1><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]))));
         LAUNCH(k_fem_restrict<float><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.rs, C.xs));
     }
     const int cc = cycle_f32(l + 1, st);
     const float *xc = cc ? C.ress : C.xs;
-    if (kind == MG_MAC) LAUNCH(k_mac_prolong<float><<<gf, blk3(), 0, st>>>(fd, cd, xb[cur], xc));
-    else LAUNCH(k_fem_prolong<float><<<gf, blk3(), 0, st>>>(fd, cd, xb[cur], xc));
+    if (kind == MG_MAC) LAUNCH(k_mac_prolong<float><<<grid_prolong(F, C), blk3(), 0, st>>>(fd, cd, xb[cur], xc));
+    else LAUNCH(k_fem_prolong<float><<<grid_prolong(F, C), blk3(), 0, st>>>(fd, cd, xb[cur], xc));
     return smooth_f32(l, v_up, cur, st);
 }
 
@@ -687,12 +698,11 @@ int mg_solver::cycle_f32(int l, cudaStream_t st) {
 void mg_solver::refine_step(cudaStream_t st) {
     mg_level &F = lv[0];
     lvl_dev fd = dev_of(F);
-    dim3 gf = grid3(F.n[0], F.n[1], F.n[2]);
     size_t n = F.npts();
-    unsigned nb = (unsigned)((n + 255) / 256);
+    unsigned nb = (unsigned)((n + 511) / 512);
     // FP64 residual -> FP32 right-hand side, FP32 start value zero (one pass)
-    if (kind == MG_MAC) LAUNCH((k_resid_to_f32<0><<<gf, blk3(), 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs)));
-    else LAUNCH((k_resid_to_f32<1><<<gf, blk3(), 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs)));
+    if (kind == MG_MAC) LAUNCH((k_resid_to_f32<0><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]))));
+    else LAUNCH((k_resid_to_f32<1><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]))));
     const int cur = cycle_f32(0, st);
     LAUNCH(k_add_f32<<<nb, 256, 0, st>>>(F.x, cur ? F.ress : F.xs, n));
 }
@@ -727,18 +737,11 @@ __global__ void k_mg_begin(mg_ctl *c, unsigned long long *mx, cudaGraphCondition
 // max |r| of the right-hand side into mx[1] (ordered bits), for the mixed
 // form's relative tolerance
 __global__ void k_absmax(const double *__restrict__ r, size_t n, unsigned long long *mx) {
-    double a = 0;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const double v = fabs(r[i]);
-        if (v != v || v > a) a = (v != v) ? __longlong_as_double(0x7ff8000000000000LL) : v;
-    }
-    unsigned long long b = (unsigned long long)__double_as_longlong(a);
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(0xffffffffu, b, o);
-        b = t > b ? t : b;
-    }
-    if ((threadIdx.x & 31) == 0) atomicMax(mx + 1, b);
+    block_max_into(body_absmax(r, n, blockIdx.x * (size_t)blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x), mx + 1);
 }
+// blocks of 256 threads for n values: enough to fill the device, at least
+// four values a thread
+static int absmax_blocks(size_t n) { return (int)std::min<size_t>((n + 1023) / 1024, 148 * 8); }
 
 __global__ void k_mg_ctl(mg_ctl *c, unsigned long long *mx, double tol, double rtol, int exact,
                          cudaGraphConditionalHandle h, int armed) {
@@ -752,9 +755,8 @@ void mg_solver::launch_body(cudaStream_t st, bool armed, unsigned long long h) {
     iterate(st);
     mg_level &F = lv[0];
     lvl_dev fd = dev_of(F);
-    dim3 gf = grid3(F.n[0], F.n[1], F.n[2]);
-    if (kind == MG_MAC) LAUNCH((k_resid_ctl<0><<<gf, blk3(), 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl)));
-    else LAUNCH((k_resid_ctl<1><<<gf, blk3(), 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl)));
+    if (kind == MG_MAC) LAUNCH((k_resid_ctl<0><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]))));
+    else LAUNCH((k_resid_ctl<1><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]))));
     LAUNCH(k_mg_ctl<<<1, 1, 0, st>>>(ctl, d_max, max_norm_tol, rtol, exact ? 1 : 0, h, armed ? 1 : 0));
 }
 
@@ -770,7 +772,7 @@ int mg_solver::capture_solve(cudaStream_t cur, graph_builder &gb) {
     cudaGraphConditionalHandle h = gb.handle(cur);
     if (gb.err != cudaSuccess) return -1;
     k_mg_begin<<<1, 1, 0, cur>>>(ctl, d_max, h, 1);
-    if (rtol > 0) k_absmax<<<148, 256, 0, cur>>>(lv[0].r, lv[0].npts(), d_max);
+    if (rtol > 0) k_absmax<<<absmax_blocks(lv[0].npts()), 256, 0, cur>>>(lv[0].r, lv[0].npts(), d_max);
     cudaStream_t body = gb.open(cur, h, cudaGraphCondTypeWhile);
     if (!body) return -1;
     long long n = 0, *saved = launches;
@@ -829,7 +831,7 @@ double mg_solver::run(cudaStream_t st) {
         k_mg_begin<<<1, 1, 0, st>>>(ctl, d_max, 0, 0);
         if (launches) (*launches)++;
         if (rtol > 0) {
-            k_absmax<<<148, 256, 0, st>>>(lv[0].r, lv[0].npts(), d_max);
+            k_absmax<<<absmax_blocks(lv[0].npts()), 256, 0, st>>>(lv[0].r, lv[0].npts(), d_max);
             if (launches) (*launches)++;
         }
         for (int guard = 0; guard < kMgMaxCycles; guard++) {

@@ -11,6 +11,7 @@
 // others continue (run[b]).  The graph WHILE loop repeats while any scene of
 // the group is still running; each scene's number of cycles is exactly its
 // solo number.
+#include <algorithm>
 #include <cstring>
 
 #include "graph_build.h"
@@ -28,38 +29,39 @@ namespace rmt3d {
     const int b_ = blockIdx.z / (zb);             \
     if (!run[b_]) return;                         \
     const int bz_ = blockIdx.z - b_ * (zb);
+// phases along the planes' lines (mg_body.cuh): blockIdx.y the plane,
+// blockIdx.z the scene
+#define MGB_LINE                                  \
+    const int b_ = blockIdx.z;                    \
+    if (!run[b_]) return;
 
 template <typename T>
-__global__ void k_mac_rb_b(lvl_dev L, T *const *x, T *const *r, const T *const *ri, int colour, const int *run,
-                           int zb) {
-    MGB_SCENE(zb)
-    body_mac_rb<T>(L, x[b_], r[b_], colour, ri ? ri[b_] : nullptr, blockIdx.x, blockIdx.y, bz_);
+__global__ void __launch_bounds__(256) k_mac_rb_b(lvl_dev L, T *const *x, T *const *r, const T *const *ri, int colour,
+                                                  const int *run, unsigned inv) {
+    MGB_LINE
+    body_mac_rb<T>(L, x[b_], r[b_], colour, ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
-// FP32: at most 51 registers, five 256-thread blocks per SM; FP64 keeps
-// four (64 registers; its stencil state spills at 51)
 template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) k_fem_gs_b(lvl_dev L, T *const *x, T *const *r, const T *const *ri, int colour, const int *run,
-                           int zb) {
-    MGB_SCENE(zb)
-    body_fem_gs<T>(L, x[b_], r[b_], colour, ri ? ri[b_] : nullptr, blockIdx.x, blockIdx.y, bz_);
+__global__ void __launch_bounds__(256) k_fem_gs_b(lvl_dev L, T *const *x, T *const *r, const T *const *ri, int colour,
+                                                  const int *run, unsigned inv) {
+    MGB_LINE
+    body_fem_gs<T>(L, x[b_], r[b_], colour, ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
 template <typename T, int KIND>
-__global__ void k_resid_b(lvl_dev L, T *const *x, T *const *r, T *const *res, const T *const *ri,
-                          unsigned long long *const *mx, const int *run, int zb) {
-    MGB_SCENE(zb)
-    const double a = body_resid<T, KIND>(L, x[b_], r[b_], res ? res[b_] : nullptr, ri ? ri[b_] : nullptr,
-                                         blockIdx.x, blockIdx.y, bz_);
-    if (mx) warp_max_into(a, mx[b_]);
+__global__ void __launch_bounds__(256) k_resid_b(lvl_dev L, T *const *x, T *const *r, T *const *res,
+                                                 const T *const *ri, const int *run, unsigned inv) {
+    MGB_LINE
+    body_resid<T, KIND>(L, x[b_], r[b_], res[b_], ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
 // the control's residual: only for scenes whose control will read it
 template <int KIND>
-__global__ void k_resid_ctl_b(lvl_dev L, double *const *x, double *const *r, const double *const *ri,
-                              unsigned long long *const *mx, mg_ctl *const *ctl, const int *run, int zb) {
-    MGB_SCENE(zb)
+__global__ void __launch_bounds__(256) k_resid_ctl_b(lvl_dev L, double *const *x, double *const *r,
+                                                     const double *const *ri, unsigned long long *const *mx,
+                                                     mg_ctl *const *ctl, const int *run, unsigned inv) {
+    MGB_LINE
     if (!ctl[b_]->need_res) return;
-    const double a = body_resid<double, KIND>(L, x[b_], r[b_], nullptr, ri ? ri[b_] : nullptr, blockIdx.x,
-                                              blockIdx.y, bz_);
-    warp_max_into(a, mx[b_]);
+    block_max_into(body_resid_max<KIND>(L, x[b_], r[b_], ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y),
+                   mx[b_]);
 }
 template <typename T>
 __global__ void k_mac_restrict_b(lvl_dev F, lvl_dev C, T *const *res, T *const *rc, T *const *xc, const int *run,
@@ -74,10 +76,11 @@ __global__ void k_fem_restrict_b(lvl_dev F, lvl_dev C, T *const *res, T *const *
     body_fem_restrict<T>(F, C, res[b_], rc[b_], xc[b_], blockIdx.x, blockIdx.y, bz_);
 }
 template <int KIND>
-__global__ void k_resid_to_f32_b(lvl_dev L, double *const *x, double *const *r, const double *const *ri,
-                                 float *const *rs, float *const *xs, const int *run, int zb) {
-    MGB_SCENE(zb)
-    body_resid_to_f32<KIND>(L, x[b_], r[b_], ri ? ri[b_] : nullptr, rs[b_], xs[b_], blockIdx.x, blockIdx.y, bz_);
+__global__ void __launch_bounds__(256) k_resid_to_f32_b(lvl_dev L, double *const *x, double *const *r,
+                                                        const double *const *ri, float *const *rs, float *const *xs,
+                                                        const int *run, unsigned inv) {
+    MGB_LINE
+    body_resid_to_f32<KIND>(L, x[b_], r[b_], ri ? ri[b_] : nullptr, rs[b_], xs[b_], inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
 template <typename T>
 __global__ void k_mac_prolong_b(lvl_dev F, lvl_dev C, T *const *x, T *const *xc, const int *run, int zb) {
@@ -146,18 +149,9 @@ __global__ void k_zero_b(T *const *a, size_t n, const int *run) {
 }
 __global__ void k_absmax_b(double *const *r, size_t n, unsigned long long *const *mx, const int *run) {
     if (!run[blockIdx.y]) return;
-    const double *rr = r[blockIdx.y];
-    double a = 0;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const double v = fabs(rr[i]);
-        if (v != v || v > a) a = (v != v) ? __longlong_as_double(0x7ff8000000000000LL) : v;
-    }
-    unsigned long long bb = (unsigned long long)__double_as_longlong(a);
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(0xffffffffu, bb, o);
-        bb = t > bb ? t : bb;
-    }
-    if ((threadIdx.x & 31) == 0) atomicMax(mx[blockIdx.y] + 1, bb);
+    block_max_into(body_absmax(r[blockIdx.y], n, blockIdx.x * (size_t)blockDim.x + threadIdx.x,
+                               (size_t)gridDim.x * blockDim.x),
+                   mx[blockIdx.y] + 1);
 }
 
 // arm the group's solve: the taking-part scenes start their control state;
@@ -324,18 +318,13 @@ static int smooth_b(mg_group &g, int l, int sweeps, int cur, cudaStream_t st, T 
         if (g.smoother == 1) {
             tile_sweep_b<T>(g, l, xb[cur], xb[cur ^ 1], r, ri, st);
             cur ^= 1;
-        } else if (g.kind == MG_MAC) {
-            int zb = (L.n[2] + 1) / 2;
-            dim3 gr((L.n[0] / 2 + 1 + 31) / 32, (L.n[1] + 3) / 4, zb * g.B);
-            for (int c = 0; c < 2; c++) {
-                k_mac_rb_b<T><<<gr, gblk(), 0, st>>>(d, xb[cur], r, ri, c, g.run, zb);
-                g.body_kernels++;
-            }
         } else {
-            int zb = (L.n[2] + 1) / 2;
-            dim3 gr(((L.n[0] + 1) / 2 + 31) / 32, ((L.n[1] + 1) / 2 + 3) / 4, zb * g.B);
-            for (int c = 0; c < 4; c++) {
-                k_fem_gs_b<T><<<gr, gblk(), 0, st>>>(d, xb[cur], r, ri, c, g.run, zb);
+            const bool mac = g.kind == MG_MAC;
+            const int rows = mac ? L.n[1] : (L.n[1] + 1) / 2, h = (L.n[0] + 1) / 2;
+            const dim3 gr((h * rows + 255) / 256, L.n[2], g.B);
+            for (int c = 0; c < (mac ? 2 : 4); c++) {
+                if (mac) k_mac_rb_b<T><<<gr, 256, 0, st>>>(d, xb[cur], r, ri, c, g.run, line_inv(h));
+                else k_fem_gs_b<T><<<gr, 256, 0, st>>>(d, xb[cur], r, ri, c, g.run, line_inv(h));
                 g.body_kernels++;
             }
         }
@@ -376,12 +365,13 @@ static int cycle_b(mg_group &g, int l, cudaStream_t st) {
     int cur = smooth_b<T>(g, l, g.v_down, 0, st, xb, Rr(l), RI(l));
     const mg_level &C = g.lv[l + 1];
     int zbf, zbc;
-    const dim3 gf = ggrid(F.n[0], F.n[1], F.n[2], g.B, zbf), gc = ggrid(C.n[0], C.n[1], C.n[2], g.B, zbc);
+    const dim3 gr((F.n[0] * F.n[1] + 255) / 256, F.n[2], g.B),
+               gf = ggrid(F.n[0], C.n[1], C.n[2], g.B, zbf), gc = ggrid(C.n[0], C.n[1], C.n[2], g.B, zbc);
     if (g.kind == MG_MAC) {
-        k_resid_b<T, 0><<<gf, gblk(), 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), nullptr, g.run, zbf);
+        k_resid_b<T, 0><<<gr, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]));
         k_mac_restrict_b<T><<<gc, gblk(), 0, st>>>(ldv(F), ldv(C), xb[cur ^ 1], Rr(l + 1), X(l + 1), g.run, zbc);
     } else {
-        k_resid_b<T, 1><<<gf, gblk(), 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), nullptr, g.run, zbf);
+        k_resid_b<T, 1><<<gr, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]));
         k_fem_restrict_b<T><<<gc, gblk(), 0, st>>>(ldv(F), ldv(C), xb[cur ^ 1], Rr(l + 1), X(l + 1), g.run, zbc);
     }
     g.body_kernels += 2;
@@ -406,15 +396,14 @@ void mg_group::iterate(cudaStream_t st) {
         return;
     }
     const mg_level &F = lv[0];
-    int zbf;
-    const dim3 gf = ggrid(F.n[0], F.n[1], F.n[2], B, zbf);
+    const dim3 gf((F.n[0] * F.n[1] + 255) / 256, F.n[2], B);
     const size_t n = F.npts();
-    const dim3 g1((unsigned)((n + 255) / 256), B);
+    const dim3 g1((unsigned)((n + 511) / 512), B);
     // FP64 residual -> FP32 right-hand side, FP32 start value zero (one pass)
     if (kind == MG_MAC)
-        k_resid_to_f32_b<0><<<gf, gblk(), 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, zbf);
+        k_resid_to_f32_b<0><<<gf, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]));
     else
-        k_resid_to_f32_b<1><<<gf, gblk(), 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, zbf);
+        k_resid_to_f32_b<1><<<gf, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]));
     body_kernels++;
     const int cur = cycle_b<float>(*this, 0, st);
     k_add_f32_b<<<g1, 256, 0, st>>>(tab[0].x, cur ? tab[0].ress : tab[0].xs, n, run);
@@ -427,7 +416,7 @@ int mg_group::capture(cudaStream_t cur, graph_builder &gb) {
     k_mgb_begin<<<1, 1024, 0, cur>>>(ctls, mx, part, run, B, h);
     outside_kernels = 1;
     if (rtol > 0) {
-        k_absmax_b<<<dim3(148, B), 256, 0, cur>>>(tab[0].r, lv[0].npts(), mx, run);
+        k_absmax_b<<<dim3((unsigned)std::min<size_t>((lv[0].npts() + 1023) / 1024, 148 * 8), B), 256, 0, cur>>>(tab[0].r, lv[0].npts(), mx, run);
         outside_kernels = 2;
     }
     cudaStream_t body = gb.open(cur, h, cudaGraphCondTypeWhile);
@@ -435,12 +424,11 @@ int mg_group::capture(cudaStream_t cur, graph_builder &gb) {
     body_kernels = 0;
     iterate(body);
     const mg_level &F = lv[0];
-    int zbf;
-    const dim3 gf = ggrid(F.n[0], F.n[1], F.n[2], B, zbf);
+    const dim3 gf((F.n[0] * F.n[1] + 255) / 256, F.n[2], B);
     if (kind == MG_MAC)
-        k_resid_ctl_b<0><<<gf, gblk(), 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, zbf);
+        k_resid_ctl_b<0><<<gf, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]));
     else
-        k_resid_ctl_b<1><<<gf, gblk(), 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, zbf);
+        k_resid_ctl_b<1><<<gf, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]));
     k_mgb_ctl<<<1, 1024, 0, body>>>(ctls, mx, run, B, tol, rtol, exact ? 1 : 0, h);
     body_kernels += 2;
     gb.close(body);

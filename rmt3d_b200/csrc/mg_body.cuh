@@ -10,31 +10,39 @@
 
 namespace rmt3d {
 
+// A phase over a level runs blocks of 256 threads along each plane's points
+// taken as one line (rows are 9 to 193 points: a block of whole rows would
+// leave up to half its lanes idle), one plane per block row.  pt: the point's
+// position on the line; split into row and column by the reciprocal
+// inv = ceil(2^31 / n), exact while (2 pt + 1) n < 2^31.  With the rim in the
+// interior's path (mg_ops.cuh), against 32 x 4 x 2 blocks and a separate rim
+// path, on a B200: FP32 FEM colour pass of the 97^3 variable-density levels
+// 9.2 -> 3.9 us, of 193^3 and 97^3 16.5 -> 11.8 us, FP64 of 65^3 4.9 -> 3.3 us.
+__host__ __device__ __forceinline__ unsigned line_inv(int n) { return (unsigned)((0x80000000ull + n - 1) / n); }
+__device__ __forceinline__ int line_row(int pt, unsigned inv) { return (int)__umulhi((unsigned)(2 * pt + 1), inv); }
+
 // ---- smoothing -------------------------------------------------------------
 template <typename T>
-__device__ __forceinline__ void body_mac_rb(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour, const T *__restrict__ ri, int bx_, int by_, int bz_) {
-    int hi = bx_ * blockDim.x + threadIdx.x;
-    int j = by_ * blockDim.y + threadIdx.y;
-    int k = bz_ * blockDim.z + threadIdx.z;
-    if (j >= L.n1 || k >= L.n2) return;
-    int i = 2 * hi + ((j + k + colour) & 1);
-    if (i >= L.n0) return;
+__device__ __forceinline__ void body_mac_rb(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour, const T *__restrict__ ri, unsigned inv, int pt, int k) {
+    const int h = (L.n0 + 1) >> 1, j = line_row(pt, inv);
+    const int i = 2 * (pt - j * h) + ((j + k + colour) & 1);
+    if (j >= L.n1 || i >= L.n0) return;
     T diag;
-    T s = ri ? mac_offdiag_vd(L, x, ri, i, j, k, diag) : mac_offdiag(L, x, i, j, k, diag);
-    int id = i + L.n0 * (j + L.n1 * k);
+    const T s = ri ? mac_offdiag_vd(L, x, ri, i, j, k, diag) : mac_offdiag(L, x, i, j, k, diag);
+    const int id = i + L.n0 * (j + L.n1 * k);
     x[id] = (r[id] - s) / diag;
 }
 
 // The Q1 stencil couples a node only to its edge and corner neighbours (the
 // face entries are zero), so colouring by the parities of i and j alone never
 // puts two coupled nodes in one colour: four colour passes are an exact
-// Gauss-Seidel sweep.
+// Gauss-Seidel sweep.  The line of a colour has (n0 + 1) / 2 nodes a row for
+// either parity of i.
 template <typename T>
-__device__ __forceinline__ void body_fem_gs(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour, const T *__restrict__ ri, int bx_, int by_, int bz_) {
-    int i = 2 * (bx_ * blockDim.x + threadIdx.x) + (colour & 1);
-    int j = 2 * (by_ * blockDim.y + threadIdx.y) + ((colour >> 1) & 1);
-    int k = bz_ * blockDim.z + threadIdx.z;
-    if (i >= L.n0 || j >= L.n1 || k >= L.n2) return;
+__device__ __forceinline__ void body_fem_gs(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour, const T *__restrict__ ri, unsigned inv, int pt, int k) {
+    const int h = (L.n0 + 1) >> 1, b = line_row(pt, inv);
+    const int i = 2 * (pt - b * h) + (colour & 1), j = 2 * b + (colour >> 1);
+    if (i >= L.n0 || j >= L.n1) return;
     T diag;
     const int id = i + L.n0 * (j + L.n1 * k);
     if (ri) {
@@ -46,56 +54,88 @@ __device__ __forceinline__ void body_fem_gs(lvl_dev L, T *__restrict__ x, const 
     }
 }
 
-// residual res = r - A x, and max |res| into *mx (as ordered bit pattern)
+// ---- residuals: r - A x into emit(index, value) ------------------------------
+template <typename T, int KIND, typename F>
+__device__ __forceinline__ void body_resid_emit(const lvl_dev &L, const T *__restrict__ x, const T *__restrict__ r,
+                                                const T *__restrict__ ri, unsigned inv, int pt, int k, F emit) {
+    const int j = line_row(pt, inv), i = pt - j * L.n0;
+    if (j >= L.n1) return;
+    T diag;
+    const T s = op_offdiag<T>(KIND, L, x, ri, i, j, k, diag);
+    const int id = i + L.n0 * (j + L.n1 * k);
+    emit(id, r[id] - s - diag * x[id]);
+}
+
+// res = r - A x
 template <typename T, int KIND>
-__device__ __forceinline__ double body_resid(lvl_dev L, const T *__restrict__ x, const T *__restrict__ r,
-                                             T *__restrict__ res, const T *__restrict__ ri, int bx_, int by_,
-                                             int bz_) {
-    int i = bx_ * blockDim.x + threadIdx.x;
-    int j = by_ * blockDim.y + threadIdx.y;
-    int k = bz_ * blockDim.z + threadIdx.z;
-    double a = 0;
-    if (i < L.n0 && j < L.n1 && k < L.n2) {
-        T diag;
-        T s = op_offdiag<T>(KIND, L, x, ri, i, j, k, diag);
-        int id = i + L.n0 * (j + L.n1 * k);
-        T v = r[id] - s - diag * x[id];
-        if (res) res[id] = v;
-        a = fabs((double)v);
-        if (a != a) a = __longlong_as_double(0x7ff8000000000000LL);
-    }
-    return a;
+__device__ __forceinline__ void body_resid(lvl_dev L, const T *__restrict__ x, const T *__restrict__ r,
+                                           T *__restrict__ res, const T *__restrict__ ri, unsigned inv, int pt, int k) {
+    body_resid_emit<T, KIND>(L, x, r, ri, inv, pt, k, [&](int id, T v) { res[id] = v; });
+}
+
+// max |r - A x| over the calling thread's points, as the ordered bit pattern
+// (NaN the largest)
+template <int KIND>
+__device__ __forceinline__ unsigned long long body_resid_max(lvl_dev L, const double *__restrict__ x,
+                                                             const double *__restrict__ r,
+                                                             const double *__restrict__ ri, unsigned inv, int pt,
+                                                             int k) {
+    unsigned long long m = 0;
+    body_resid_emit<double, KIND>(L, x, r, ri, inv, pt, k, [&](int, double v) {
+        const double a = fabs(v);
+        const unsigned long long b = a != a ? 0x7ff8000000000000ULL : (unsigned long long)__double_as_longlong(a);
+        m = b > m ? b : m;
+    });
+    return m;
 }
 
 // The mixed form's FP64 residual handed to the FP32 cycle in one pass: the
-// residual r - A x in FP64 (body_resid's expression), rounded to FP32 as the
-// cycle's right-hand side, and the cycle's FP32 start value zeroed.
+// residual r - A x in FP64, rounded to FP32 as the cycle's right-hand side,
+// and the cycle's FP32 start value zeroed.
 template <int KIND>
 __device__ __forceinline__ void body_resid_to_f32(lvl_dev L, const double *__restrict__ x,
                                                   const double *__restrict__ r, const double *__restrict__ ri,
-                                                  float *__restrict__ rs, float *__restrict__ xs, int bx_, int by_,
-                                                  int bz_) {
-    int i = bx_ * blockDim.x + threadIdx.x;
-    int j = by_ * blockDim.y + threadIdx.y;
-    int k = bz_ * blockDim.z + threadIdx.z;
-    if (i >= L.n0 || j >= L.n1 || k >= L.n2) return;
-    double diag;
-    const double s = op_offdiag<double>(KIND, L, x, ri, i, j, k, diag);
-    const int id = i + L.n0 * (j + L.n1 * k);
-    const double v = r[id] - s - diag * x[id];
-    rs[id] = (float)v;
-    xs[id] = 0;
+                                                  float *__restrict__ rs, float *__restrict__ xs, unsigned inv,
+                                                  int pt, int k) {
+    body_resid_emit<double, KIND>(L, x, r, ri, inv, pt, k, [&](int id, double v) {
+        rs[id] = (float)v;
+        xs[id] = 0;
+    });
 }
 
-// max of a (non-negative, NaN sticky as the largest bit pattern) over the
-// block's warps into *mx
-__device__ __forceinline__ void warp_max_into(double a, unsigned long long *mx) {
-    unsigned long long b = (unsigned long long)__double_as_longlong(a);
+// the block's maximum of b into *mx: one atomic per block, none where the
+// maximum so far already covers it (an atomic per warp made the 192^3 MAC norm
+// 63 us; now 31).  Every thread of the block calls it.
+__device__ __forceinline__ void block_max_into(unsigned long long b, unsigned long long *mx) {
+    __shared__ unsigned long long wmax[32];
     for (int o = 16; o > 0; o >>= 1) {
-        unsigned long long t = __shfl_xor_sync(0xffffffffu, b, o);
+        const unsigned long long t = __shfl_xor_sync(0xffffffffu, b, o);
         b = t > b ? t : b;
     }
-    if ((threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) % 32 == 0) atomicMax(mx, b);
+    const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+    const int nw = (blockDim.x * blockDim.y * blockDim.z) >> 5;
+    if ((tid & 31) == 0) wmax[tid >> 5] = b;
+    __syncthreads();
+    if (tid < 32) {
+        b = tid < nw ? wmax[tid] : 0;
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long t = __shfl_xor_sync(0xffffffffu, b, o);
+            b = t > b ? t : b;
+        }
+        if (tid == 0 && b > *(volatile unsigned long long *)mx) atomicMax(mx, b);
+    }
+}
+
+// max |r| over a grid-stride range, as the ordered bit pattern (NaN the largest)
+__device__ __forceinline__ unsigned long long body_absmax(const double *__restrict__ r, size_t n, size_t t0, size_t ts) {
+    unsigned long long m = 0;
+#pragma unroll 4
+    for (size_t i = t0; i < n; i += ts) {
+        const double a = fabs(r[i]);
+        const unsigned long long b = a != a ? 0x7ff8000000000000ULL : (unsigned long long)__double_as_longlong(a);
+        m = b > m ? b : m;
+    }
+    return m;
 }
 
 // ---- grid transfer ---------------------------------------------------------
@@ -114,38 +154,62 @@ __device__ __forceinline__ void body_mac_restrict(lvl_dev F, lvl_dev C, const T 
     xc0[I + C.n0 * (J + C.n1 * K)] = 0;
 }
 
+// x += the interpolated coarse correction.  A thread takes the 2 x 2 fine
+// points (j, k) around one pair of coarse rows at its i: they share their
+// coarse values (18 loads for four points instead of 32; FEM 8 instead of up
+// to 27), and each point's sum keeps its order.  FEM, 193^3 and 97^3 levels:
+// 101 -> 15 us a launch; its DRAM floor is 9 us.
 template <typename T>
 __device__ __forceinline__ void body_mac_prolong(lvl_dev F, lvl_dev C, T *__restrict__ x, const T *__restrict__ xc, int bx_, int by_, int bz_) {
-    int i = bx_ * blockDim.x + threadIdx.x;
-    int j = by_ * blockDim.y + threadIdx.y;
-    int k = bz_ * blockDim.z + threadIdx.z;
-    if (i >= F.n0 || j >= F.n1 || k >= F.n2) return;
-    const int f[3] = {i, j, k};
-    const int nc[3] = {C.n0, C.n1, C.n2}, p[3] = {C.p0, C.p1, C.p2};
-    int ci[3][2];
-    T w[3][2];
-    for (int d = 0; d < 3; d++) {
-        int I = f[d] >> 1;
-        int J = wrapi(I + ((f[d] & 1) ? 1 : -1), nc[d], p[d]);
-        ci[d][0] = I;
-        if (J < 0) {
-            w[d][0] = 1;
-            ci[d][1] = I;
-            w[d][1] = 0;
-        } else {
-            w[d][0] = (T)0.75;
-            ci[d][1] = J;
-            w[d][1] = (T)0.25;
+    const int i = bx_ * blockDim.x + threadIdx.x;
+    const int J = by_ * blockDim.y + threadIdx.y;
+    const int K = bz_ * blockDim.z + threadIdx.z;
+    if (i >= F.n0 || J >= C.n1 || K >= C.n2) return;
+    const int I = i >> 1, In = wrapi(I + ((i & 1) ? 1 : -1), C.n0, C.p0);
+    const T wx[2] = {In < 0 ? (T)1 : (T)0.75, In < 0 ? (T)0 : (T)0.25};
+    const int ix = In < 0 ? I : In;
+    int jy[3], kz[3];
+    bool oy[3], oz[3];
+#pragma unroll
+    for (int o = 0; o < 3; o++) {
+        const int a = wrapi(J + o - 1, C.n1, C.p1), b = wrapi(K + o - 1, C.n2, C.p2);
+        oy[o] = a >= 0;
+        oz[o] = b >= 0;
+        jy[o] = a < 0 ? J : a;
+        kz[o] = b < 0 ? K : b;
+    }
+    T v[3][3][2];
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const T *row = xc + (size_t)C.n0 * (jy[b] + (size_t)C.n1 * kz[c]);
+            v[c][b][0] = row[I];
+            v[c][b][1] = row[ix];
+        }
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const int k = 2 * K + c;
+        if (k >= F.n2) continue;
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const int j = 2 * J + b;
+            if (j >= F.n1) continue;
+            // odd points lean on the next coarse cell, even ones on the
+            // previous; without it the near cell counts fully
+            const int nb = b ? 2 : 0, nc = c ? 2 : 0;
+            const T wy[2] = {oy[nb] ? (T)0.75 : (T)1, oy[nb] ? (T)0.25 : (T)0};
+            const T wz[2] = {oz[nc] ? (T)0.75 : (T)1, oz[nc] ? (T)0.25 : (T)0};
+            T e = 0;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int qa = q & 1, qb = (q >> 1) & 1, qc = q >> 2;
+                const T wt = wx[qa] * wy[qb] * wz[qc];
+                if (wt != 0) e += wt * v[qc ? nc : 1][qb ? nb : 1][qa];
+            }
+            x[i + F.n0 * (j + F.n1 * k)] += e;
         }
     }
-    T e = 0;
-    for (int c = 0; c < 2; c++)
-        for (int b = 0; b < 2; b++)
-            for (int a = 0; a < 2; a++) {
-                T wt = w[0][a] * w[1][b] * w[2][c];
-                if (wt != 0) e += wt * xc[ci[0][a] + C.n0 * (ci[1][b] + C.n1 * ci[2][c])];
-            }
-    x[i + F.n0 * (j + F.n1 * k)] += e;
 }
 
 template <typename T>
@@ -182,33 +246,44 @@ __device__ __forceinline__ void body_fem_restrict(lvl_dev F, lvl_dev C, const T 
 
 template <typename T>
 __device__ __forceinline__ void body_fem_prolong(lvl_dev F, lvl_dev C, T *__restrict__ x, const T *__restrict__ xc, int bx_, int by_, int bz_) {
-    int i = bx_ * blockDim.x + threadIdx.x;
-    int j = by_ * blockDim.y + threadIdx.y;
-    int k = bz_ * blockDim.z + threadIdx.z;
-    if (i >= F.n0 || j >= F.n1 || k >= F.n2) return;
-    const int f[3] = {i, j, k};
-    const int nc[3] = {C.n0, C.n1, C.n2}, p[3] = {C.p0, C.p1, C.p2};
-    int ci[3][2];
-    T w[3][2];
-    int cnt[3];
-    for (int d = 0; d < 3; d++) {
-        if ((f[d] & 1) == 0) {
-            ci[d][0] = f[d] >> 1;
-            w[d][0] = 1;
-            cnt[d] = 1;
-        } else {
-            ci[d][0] = f[d] >> 1;
-            ci[d][1] = wrapi((f[d] >> 1) + 1, nc[d], p[d]);
-            w[d][0] = w[d][1] = (T)0.5;
-            cnt[d] = 2;
+    const int i = bx_ * blockDim.x + threadIdx.x;
+    const int J = by_ * blockDim.y + threadIdx.y;
+    const int K = bz_ * blockDim.z + threadIdx.z;
+    if (i >= F.n0 || J >= C.n1 || K >= C.n2) return;
+    const bool odd = i & 1;
+    const int I = i >> 1, I1 = odd ? wrapi(I + 1, C.n0, C.p0) : I;
+    // beyond a wall there is no point that would use the next row or plane
+    const int J1 = max(wrapi(J + 1, C.n1, C.p1), 0), K1 = max(wrapi(K + 1, C.n2, C.p2), 0);
+    const T wx = odd ? (T)0.5 : (T)1;
+    T v[2][2][2];
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const T *row = xc + (size_t)C.n0 * ((b ? J1 : J) + (size_t)C.n1 * (c ? K1 : K));
+            v[c][b][0] = row[I];
+            v[c][b][1] = row[I1];
+        }
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const int k = 2 * K + c;
+        if (k >= F.n2) continue;
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const int j = 2 * J + b;
+            if (j >= F.n1) continue;
+            const T w = wx * (b ? (T)0.5 : (T)1) * (c ? (T)0.5 : (T)1);
+            T e = 0;
+#pragma unroll
+            for (int qc = 0; qc <= c; qc++)
+#pragma unroll
+                for (int qb = 0; qb <= b; qb++) {
+                    e += w * v[qc][qb][0];
+                    if (odd) e += w * v[qc][qb][1];
+                }
+            x[i + F.n0 * (j + F.n1 * k)] += e;
         }
     }
-    T e = 0;
-    for (int c = 0; c < cnt[2]; c++)
-        for (int b = 0; b < cnt[1]; b++)
-            for (int a = 0; a < cnt[0]; a++)
-                e += w[0][a] * w[1][b] * w[2][c] * xc[ci[0][a] + C.n0 * (ci[1][b] + C.n1 * ci[2][c])];
-    x[i + F.n0 * (j + F.n1 * k)] += e;
 }
 
 // coarsest grid: x = B r with the precomputed dense inverse B (row-major)
@@ -254,9 +329,18 @@ __device__ __forceinline__ void body_to_f32(const double *__restrict__ a, float 
     size_t i = bx_ * (size_t)blockDim.x + threadIdx.x;
     if (i < n) b[i] = (float)a[i];
 }
+// two elements a thread (the level arrays start on 256-byte boundaries)
 __device__ __forceinline__ void body_add_f32(double *__restrict__ a, const float *__restrict__ b, size_t n, int bx_) {
-    size_t i = bx_ * (size_t)blockDim.x + threadIdx.x;
-    if (i < n) a[i] += (double)b[i];
+    const size_t i = 2 * (bx_ * (size_t)blockDim.x + threadIdx.x);
+    if (i + 1 < n) {
+        double2 v = *reinterpret_cast<double2 *>(a + i);
+        const float2 w = *reinterpret_cast<const float2 *>(b + i);
+        v.x += (double)w.x;
+        v.y += (double)w.y;
+        *reinterpret_cast<double2 *>(a + i) = v;
+    } else if (i < n) {
+        a[i] += (double)b[i];
+    }
 }
 template <typename T>
 __device__ __forceinline__ void body_zero(T *a, size_t n, int bx_) {

@@ -27,82 +27,99 @@ __device__ __forceinline__ T div_pow2(T v, int num) {
 }
 
 // ---- operator application -------------------------------------------------
+// The sum of the off-diagonal terms of one row and its diagonal.  Interior
+// and rim points load the same neighbours (a missing one's place is taken by
+// any stored value), so a warp that holds the end of a row loads once: rim
+// points, about one in every warp of a 64^3 level, then only sum in another
+// way -- term by term, missing neighbours with coefficient zero, whose terms
+// leave the sum's bits alone.
+
+// offsets to the lower and upper neighbour along an axis of n >= 2 points
+// (stride st): the image across a periodic seam; beyond a wall the neighbour
+// on the other side stands in (never a point of the same colour, so nothing
+// that a colour pass is writing is read)
+__device__ __forceinline__ int nb_lo(int c, int n, int prd, int st) { return c > 0 ? -st : (prd ? (n - 1) * st : st); }
+__device__ __forceinline__ int nb_hi(int c, int n, int prd, int st) { return c < n - 1 ? st : (prd ? (1 - n) * st : -st); }
+
 template <typename T>
 __device__ __forceinline__ T mac_offdiag(const lvl_dev L, const T *__restrict__ x, int i, int j, int k, T &diag) {
+    const int sy = L.n0, sz = L.n0 * L.n1;
+    const T *c = x + i + sy * j + sz * k;
+    T xm = c[nb_lo(i, L.n0, L.p0, 1)], xp = c[nb_hi(i, L.n0, L.p0, 1)];
+    T ym = c[nb_lo(j, L.n1, L.p1, sy)], yp = c[nb_hi(j, L.n1, L.p1, sy)];
+    T zm = c[nb_lo(k, L.n2, L.p2, sz)], zp = c[nb_hi(k, L.n2, L.p2, sz)];
     if (i > 0 && i < L.n0 - 1 && j > 0 && j < L.n1 - 1 && k > 0 && k < L.n2 - 1) {
-        const int sy = L.n0, sz = L.n0 * L.n1;
-        const T *c = x + i + sy * j + sz * k;
         diag = (T)-6;
-        return ((c[-1] + c[1]) + (c[-sy] + c[sy])) + (c[-sz] + c[sz]);
+        return ((xm + xp) + (ym + yp)) + (zm + zp);
     }
+    const bool a0 = i == 0 && !L.p0, a1 = i == L.n0 - 1 && !L.p0, b0 = j == 0 && !L.p1, b1 = j == L.n1 - 1 && !L.p1,
+               c0 = k == 0 && !L.p2, c1 = k == L.n2 - 1 && !L.p2;
     T s = 0;
-    int missing = 0;
-    const int n[3] = {L.n0, L.n1, L.n2}, p[3] = {L.p0, L.p1, L.p2};
-    const int c[3] = {i, j, k};
-    const int st[3] = {1, L.n0, L.n0 * L.n1};
-    const int base = i + L.n0 * (j + L.n1 * k);
-    for (int d = 0; d < 3; d++) {
-        for (int sgn = -1; sgn <= 1; sgn += 2) {
-            int v = wrapi(c[d] + sgn, n[d], p[d]);
-            if (v < 0) {
-                missing++;
-                continue;
-            }
-            s += x[base + (v - c[d]) * st[d]];
-        }
-    }
-    diag = (T)(-6 + missing);
+    s += a0 ? (T)0 : xm;
+    s += a1 ? (T)0 : xp;
+    s += b0 ? (T)0 : ym;
+    s += b1 ? (T)0 : yp;
+    s += c0 ? (T)0 : zm;
+    s += c1 ? (T)0 : zp;
+    diag = (T)(-6 + (int)a0 + (int)a1 + (int)b0 + (int)b1 + (int)c0 + (int)c1);
     return s;
 }
 
 template <typename T>
 __device__ __forceinline__ T fem_offdiag(const lvl_dev L, const T *__restrict__ x, int i, int j, int k, T &diag) {
+    // edges -2, corners -1, faces 0
+    const int sy = L.n0, sz = L.n0 * L.n1;
+    const int xl = nb_lo(i, L.n0, L.p0, 1), xh = nb_hi(i, L.n0, L.p0, 1);
+    const T *c = x + i + sy * j + sz * k;
+    const T *y0 = c + nb_lo(j, L.n1, L.p1, sy), *y2 = c + nb_hi(j, L.n1, L.p1, sy);
+    const int zl = nb_lo(k, L.n2, L.p2, sz), zh = nb_hi(k, L.n2, L.p2, sz);
+    const T a00 = y0[zl + xl], a10 = y0[zl], a20 = y0[zl + xh], a01 = c[zl + xl], a21 = c[zl + xh], a02 = y2[zl + xl],
+            a12 = y2[zl], a22 = y2[zl + xh];
+    const T b00 = y0[xl], b20 = y0[xh], b02 = y2[xl], b22 = y2[xh];
+    const T d00 = y0[zh + xl], d10 = y0[zh], d20 = y0[zh + xh], d01 = c[zh + xl], d21 = c[zh + xh], d02 = y2[zh + xl],
+            d12 = y2[zh], d22 = y2[zh + xh];
     if (i > 0 && i < L.n0 - 1 && j > 0 && j < L.n1 - 1 && k > 0 && k < L.n2 - 1) {
-        // interior node: edges -2, corners -1, faces 0
-        const int sy = L.n0, sz = L.n0 * L.n1;
-        const T *c = x + i + sy * j + sz * k;
-        const T *zm = c - sz, *zp = c + sz;
-        T e = (c[-1 - sy] + c[1 - sy]) + (c[-1 + sy] + c[1 + sy]);
-        e += (zm[-1] + zm[1]) + (zm[-sy] + zm[sy]);
-        e += (zp[-1] + zp[1]) + (zp[-sy] + zp[sy]);
-        T q = (zm[-1 - sy] + zm[1 - sy]) + (zm[-1 + sy] + zm[1 + sy]);
-        q += (zp[-1 - sy] + zp[1 - sy]) + (zp[-1 + sy] + zp[1 + sy]);
+        T e = (b00 + b20) + (b02 + b22);
+        e += (a01 + a21) + (a10 + a12);
+        e += (d01 + d21) + (d10 + d12);
+        T q = (a00 + a20) + (a02 + a22);
+        q += (d00 + d20) + (d02 + d22);
         diag = (T)32;
         return (T)-2 * e - q;
     }
-    const int n[3] = {L.n0, L.n1, L.n2}, p[3] = {L.p0, L.p1, L.p2};
-    const int c[3] = {i, j, k};
-    bool bd[3];
-    for (int d = 0; d < 3; d++) bd[d] = !p[d] && (c[d] == 0 || c[d] == n[d] - 1);
-    int nb[3][3];
-    for (int d = 0; d < 3; d++)
-        for (int o = -1; o <= 1; o++) nb[d][o + 1] = wrapi(c[d] + o, n[d], p[d]);
+    // 1 where the neighbour on that side exists; an entry is halved once per
+    // wall plane the node lies on along an axis it does not move along
+    const bool wx = !L.p0 && (i == 0 || i == L.n0 - 1), wy = !L.p1 && (j == 0 || j == L.n1 - 1),
+               wz = !L.p2 && (k == 0 || k == L.n2 - 1);
+    const T x0 = !L.p0 && i == 0 ? (T)0 : (T)1, x1 = !L.p0 && i == L.n0 - 1 ? (T)0 : (T)1;
+    const T v0 = !L.p1 && j == 0 ? (T)0 : (T)1, v1 = !L.p1 && j == L.n1 - 1 ? (T)0 : (T)1;
+    const T z0 = !L.p2 && k == 0 ? (T)0 : (T)1, z1 = !L.p2 && k == L.n2 - 1 ? (T)0 : (T)1;
+    const T ex = wx ? (T)-1 : (T)-2, ey = wy ? (T)-1 : (T)-2, ez = wz ? (T)-1 : (T)-2;
+    const T p00 = x0 * v0, p20 = x1 * v0, p02 = x0 * v1, p22 = x1 * v1;
     T s = 0;
-    for (int oc = 0; oc < 3; oc++) {
-        int kk = nb[2][oc];
-        if (kk < 0) continue;
-        for (int ob = 0; ob < 3; ob++) {
-            int jj = nb[1][ob];
-            if (jj < 0) continue;
-            const T *row = x + (size_t)L.n0 * (jj + (size_t)L.n1 * kk);
-            for (int oa = 0; oa < 3; oa++) {
-                int ii = nb[0][oa];
-                if (ii < 0) continue;
-                int nz = (oa != 1) + (ob != 1) + (oc != 1);
-                if (nz == 0 || nz == 1) continue;  // centre handled below, faces are 0
-                T co = (nz == 2) ? (T)-2 : (T)-1;
-                int halve = (bd[0] && oa == 1) + (bd[1] && ob == 1) + (bd[2] && oc == 1);
-                if (halve == 1) co *= (T)0.5;
-                else if (halve == 2) co *= (T)0.25;
-                s += co * row[ii];
-            }
-        }
-    }
-    int hc = bd[0] + bd[1] + bd[2];
-    diag = (T)32 / (T)(1 << hc);
+    s += -(p00 * z0) * a00;
+    s += ex * (v0 * z0) * a10;
+    s += -(p20 * z0) * a20;
+    s += ey * (x0 * z0) * a01;
+    s += ey * (x1 * z0) * a21;
+    s += -(p02 * z0) * a02;
+    s += ex * (v1 * z0) * a12;
+    s += -(p22 * z0) * a22;
+    s += ez * p00 * b00;
+    s += ez * p20 * b20;
+    s += ez * p02 * b02;
+    s += ez * p22 * b22;
+    s += -(p00 * z1) * d00;
+    s += ex * (v0 * z1) * d10;
+    s += -(p20 * z1) * d20;
+    s += ey * (x0 * z1) * d01;
+    s += ey * (x1 * z1) * d21;
+    s += -(p02 * z1) * d02;
+    s += ex * (v1 * z1) * d12;
+    s += -(p22 * z1) * d22;
+    diag = (T)(32 >> ((int)wx + (int)wy + (int)wz));
     return s;
 }
-
 
 // 1 / diag of the constant-density FEM stencil at node (i, j, k).  diag is
 // 32 / 2^h, h the number of walled axes on whose end planes the node lies,
@@ -127,49 +144,24 @@ __device__ __forceinline__ T fem_inv_diag(const lvl_dev L, int i, int j, int k) 
 template <typename T>
 __device__ __forceinline__ T mac_offdiag_vd(const lvl_dev L, const T *__restrict__ x, const T *__restrict__ ri, int i,
                                             int j, int k, T &diag) {
-    const int base = i + L.n0 * (j + L.n1 * k);
-    const T rc = ri[base];
-    if (i > 0 && i < L.n0 - 1 && j > 0 && j < L.n1 - 1 && k > 0 && k < L.n2 - 1) {
-        // interior cell: all six faces, the same operations in the same order
-        const int sy = L.n0, sz = L.n0 * L.n1;
-        const T ax1 = (T)0.5 * (ri[base - 1] + rc), ax2 = (T)0.5 * (rc + ri[base + 1]);
-        const T ay1 = (T)0.5 * (ri[base - sy] + rc), ay2 = (T)0.5 * (rc + ri[base + sy]);
-        const T az1 = (T)0.5 * (ri[base - sz] + rc), az2 = (T)0.5 * (rc + ri[base + sz]);
-        T s = 0, csum = 0;
-        s += ax1 * x[base - 1] + ax2 * x[base + 1];
-        csum += ax1 + ax2;
-        s += ay1 * x[base - sy] + ay2 * x[base + sy];
-        csum += ay1 + ay2;
-        s += az1 * x[base - sz] + az2 * x[base + sz];
-        csum += az1 + az2;
-        diag = (T)(-6) * (csum / (T)6);
-        return s;
-    }
-    const int n[3] = {L.n0, L.n1, L.n2}, p[3] = {L.p0, L.p1, L.p2};
-    const int c[3] = {i, j, k};
-    const int st[3] = {1, L.n0, L.n0 * L.n1};
+    const int sy = L.n0, sz = L.n0 * L.n1, base = i + sy * j + sz * k;
+    const T *c = x + base, *q = ri + base;
+    const int xl = nb_lo(i, L.n0, L.p0, 1), xh = nb_hi(i, L.n0, L.p0, 1), yl = nb_lo(j, L.n1, L.p1, sy),
+              yh = nb_hi(j, L.n1, L.p1, sy), zl = nb_lo(k, L.n2, L.p2, sz), zh = nb_hi(k, L.n2, L.p2, sz);
+    const T rc = q[0];
+    const bool a0 = i > 0 || L.p0, a1 = i < L.n0 - 1 || L.p0, b0 = j > 0 || L.p1, b1 = j < L.n1 - 1 || L.p1,
+               c0 = k > 0 || L.p2, c1 = k < L.n2 - 1 || L.p2;
+    const T ax1 = a0 ? (T)0.5 * (q[xl] + rc) : (T)0, ax2 = a1 ? (T)0.5 * (rc + q[xh]) : (T)0;
+    const T ay1 = b0 ? (T)0.5 * (q[yl] + rc) : (T)0, ay2 = b1 ? (T)0.5 * (rc + q[yh]) : (T)0;
+    const T az1 = c0 ? (T)0.5 * (q[zl] + rc) : (T)0, az2 = c1 ? (T)0.5 * (rc + q[zh]) : (T)0;
     T s = 0, csum = 0;
-    int cnt = 0;
-    for (int d = 0; d < 3; d++) {
-        const int lo = wrapi(c[d] - 1, n[d], p[d]), hi = wrapi(c[d] + 1, n[d], p[d]);
-        const int il = base + (lo - c[d]) * st[d], ih = base + (hi - c[d]) * st[d];
-        if (lo >= 0 && hi >= 0) {
-            const T a1 = (T)0.5 * (ri[il] + rc), a2 = (T)0.5 * (rc + ri[ih]);
-            s += a1 * x[il] + a2 * x[ih];
-            csum += a1 + a2;
-            cnt += 2;
-        } else if (lo >= 0) {
-            const T a1 = (T)0.5 * (ri[il] + rc);
-            s += a1 * x[il];
-            csum += a1;
-            cnt += 1;
-        } else if (hi >= 0) {
-            const T a2 = (T)0.5 * (rc + ri[ih]);
-            s += a2 * x[ih];
-            csum += a2;
-            cnt += 1;
-        }
-    }
+    s += ax1 * c[xl] + ax2 * c[xh];
+    csum += ax1 + ax2;
+    s += ay1 * c[yl] + ay2 * c[yh];
+    csum += ay1 + ay2;
+    s += az1 * c[zl] + az2 * c[zh];
+    csum += az1 + az2;
+    const int cnt = (int)a0 + (int)a1 + (int)b0 + (int)b1 + (int)c0 + (int)c1;
     diag = (T)(-cnt) * (csum / (T)cnt);
     return s;
 }
@@ -178,134 +170,57 @@ __device__ __forceinline__ T mac_offdiag_vd(const lvl_dev L, const T *__restrict
 // (boundary-halved) Q1 stencil is scaled by the mean of 1/rho over the cells
 // adjacent to both the node and that neighbour -- 1 cell for a corner
 // neighbour, 2 for an edge neighbour, all (up to 8) for the centre -- summed
-// in the reference's cell order.
+// in the reference's cell order.  With a missing cell's 1/rho as zero that is
+// -v for a corner, -(va + vb) for an edge (twice the mean of two cells, or
+// once the one cell that a wall leaves, with the entry halved) and 4 times
+// the sum for the centre, each exactly; a missing neighbour has no cells.
 template <typename T>
 __device__ __forceinline__ T fem_offdiag_vd(const lvl_dev L, const T *__restrict__ x, const T *__restrict__ ri, int i,
                                             int j, int k, T &diag) {
-    if (i > 0 && i < L.n0 - 1 && j > 0 && j < L.n1 - 1 && k > 0 && k < L.n2 - 1) {
-        // interior node (all 8 cells exist, no halving): corners take one
-        // cell, edges the mean of two (lower index first), the centre the
-        // mean of all eight in (z, y, x) order; the means multiply by 1/2 and
-        // 1/8, the same bits as the divisions without their instruction
-        // sequences
-        const int sy = L.n0, sz = L.n0 * L.n1;
-        const int ncx = L.p0 ? L.n0 : L.n0 - 1, ncy = L.p1 ? L.n1 : L.n1 - 1;
-        const int c0 = (i - 1) + ncx * ((j - 1) + ncy * (k - 1));  // cell below-left-front
-        const int cy = ncx, cz = ncx * ncy;
-        T v[2][2][2];
-        v[0][0][0] = ri[c0];
-        v[0][0][1] = ri[c0 + 1];
-        v[0][1][0] = ri[c0 + cy];
-        v[0][1][1] = ri[c0 + cy + 1];
-        v[1][0][0] = ri[c0 + cz];
-        v[1][0][1] = ri[c0 + cz + 1];
-        v[1][1][0] = ri[c0 + cz + cy];
-        v[1][1][1] = ri[c0 + cz + cy + 1];
-        const T *xc = x + i + sy * j + sz * k;
-        T s = 0;
-#pragma unroll
-        for (int oc = 0; oc < 3; oc++)
-#pragma unroll
-            for (int ob = 0; ob < 3; ob++)
-#pragma unroll
-                for (int oa = 0; oa < 3; oa++) {
-                    const int nz = (oa != 1) + (ob != 1) + (oc != 1);
-                    if (nz <= 1) continue;
-                    const T xv = xc[(oa - 1) + sy * (ob - 1) + sz * (oc - 1)];
-                    T cf;
-                    if (nz == 3) {
-                        cf = -v[oc >> 1][ob >> 1][oa >> 1];
-                    } else if (oc == 1) {
-                        cf = (T)-2 * ((v[0][ob >> 1][oa >> 1] + v[1][ob >> 1][oa >> 1]) * (T)0.5);
-                    } else if (ob == 1) {
-                        cf = (T)-2 * ((v[oc >> 1][0][oa >> 1] + v[oc >> 1][1][oa >> 1]) * (T)0.5);
-                    } else {
-                        cf = (T)-2 * ((v[oc >> 1][ob >> 1][0] + v[oc >> 1][ob >> 1][1]) * (T)0.5);
-                    }
-                    s += cf * xv;
-                }
-        T c8 = 0;
-#pragma unroll
-        for (int a = 0; a < 2; a++)
-#pragma unroll
-            for (int b = 0; b < 2; b++)
-#pragma unroll
-                for (int e = 0; e < 2; e++) c8 += v[a][b][e];
-        diag = (T)32 * (c8 * (T)0.125);
-        return s;
-    }
-    // boundary or wrapped node; every loop below unrolls to constant indices
-    const int n[3] = {L.n0, L.n1, L.n2}, p[3] = {L.p0, L.p1, L.p2};
-    const int nc[3] = {p[0] ? n[0] : n[0] - 1, p[1] ? n[1] : n[1] - 1, p[2] ? n[2] : n[2] - 1};
-    const int c[3] = {i, j, k};
-    int cell[3][2];  // cells below / above the node on each axis (-1: none)
-    bool bd[3];
-    int nb[3][3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        bd[d] = !p[d] && (c[d] == 0 || c[d] == n[d] - 1);
-        cell[d][0] = (c[d] - 1 >= 0) ? c[d] - 1 : (p[d] ? c[d] - 1 + nc[d] : -1);
-        cell[d][1] = (c[d] < nc[d]) ? c[d] : (p[d] ? c[d] - nc[d] : -1);
-#pragma unroll
-        for (int o = -1; o <= 1; o++) nb[d][o + 1] = wrapi(c[d] + o, n[d], p[d]);
-    }
-    // the up to 8 adjacent cells' 1/rho, [cz][cy][cx]
-    T v[2][2][2];
-#pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 2; b++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const bool ok = cell[0][e] >= 0 && cell[1][b] >= 0 && cell[2][a] >= 0;
-                v[a][b][e] = ok ? ri[cell[0][e] + nc[0] * (cell[1][b] + nc[1] * cell[2][a])] : (T)0;
-            }
+    const int sy = L.n0, sz = L.n0 * L.n1;
+    const int ncx = L.p0 ? L.n0 : L.n0 - 1, ncy = L.p1 ? L.n1 : L.n1 - 1, ncz = L.p2 ? L.n2 : L.n2 - 1;
+    // cells below and above the node on each axis, -1: none
+    const int i0 = i > 0 ? i - 1 : (L.p0 ? ncx - 1 : -1), i1 = i < ncx ? i : -1;
+    const int j0 = j > 0 ? j - 1 : (L.p1 ? ncy - 1 : -1), j1 = j < ncy ? j : -1;
+    const int k0 = k > 0 ? k - 1 : (L.p2 ? ncz - 1 : -1), k1 = k < ncz ? k : -1;
+    auto cell = [&](int a, int b, int c) -> T { return (a | b | c) >= 0 ? ri[a + ncx * (b + ncy * c)] : (T)0; };
+    const T u00 = cell(i0, j0, k0), u10 = cell(i1, j0, k0), u01 = cell(i0, j1, k0), u11 = cell(i1, j1, k0);
+    const T v00 = cell(i0, j0, k1), v10 = cell(i1, j0, k1), v01 = cell(i0, j1, k1), v11 = cell(i1, j1, k1);
+    const int xl = nb_lo(i, L.n0, L.p0, 1), xh = nb_hi(i, L.n0, L.p0, 1);
+    const T *c = x + i + sy * j + sz * k;
+    const T *y0 = c + nb_lo(j, L.n1, L.p1, sy), *y2 = c + nb_hi(j, L.n1, L.p1, sy);
+    const int zl = nb_lo(k, L.n2, L.p2, sz), zh = nb_hi(k, L.n2, L.p2, sz);
     T s = 0;
-#pragma unroll
-    for (int oc = 0; oc < 3; oc++) {
-#pragma unroll
-        for (int ob = 0; ob < 3; ob++) {
-#pragma unroll
-            for (int oa = 0; oa < 3; oa++) {
-                const int nz = (oa != 1) + (ob != 1) + (oc != 1);
-                if (nz <= 1) continue;  // centre handled below, faces are 0
-                const int kk = nb[2][oc], jj = nb[1][ob], ii = nb[0][oa];
-                if (kk < 0 || jj < 0 || ii < 0) continue;
-                T co = (nz == 2) ? (T)-2 : (T)-1;
-                const int halve = (bd[0] && oa == 1) + (bd[1] && ob == 1) + (bd[2] && oc == 1);
-                if (halve == 1) co *= (T)0.5;
-                else if (halve == 2) co *= (T)0.25;
-                // cells shared by the node and this neighbour, in (z, y, x) order
-                T sum = 0;
-                int num = 0;
-#pragma unroll
-                for (int a = (oc == 2 ? 1 : 0); a <= (oc == 0 ? 0 : 1); a++)
-#pragma unroll
-                    for (int b = (ob == 2 ? 1 : 0); b <= (ob == 0 ? 0 : 1); b++)
-#pragma unroll
-                        for (int e = (oa == 2 ? 1 : 0); e <= (oa == 0 ? 0 : 1); e++)
-                            if (cell[2][a] >= 0 && cell[1][b] >= 0 && cell[0][e] >= 0) {
-                                sum += v[a][b][e];
-                                num++;
-                            }
-                s += co * div_pow2(sum, num) * x[ii + L.n0 * (jj + L.n1 * kk)];
-            }
-        }
-    }
-    T sum = 0;
-    int num = 0;
-#pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 2; b++)
-#pragma unroll
-            for (int e = 0; e < 2; e++)
-                if (cell[2][a] >= 0 && cell[1][b] >= 0 && cell[0][e] >= 0) {
-                    sum += v[a][b][e];
-                    num++;
-                }
-    const int hc = bd[0] + bd[1] + bd[2];
-    diag = ((T)32 / (T)(1 << hc)) * div_pow2(sum, num);
+    s += -u00 * y0[zl + xl];
+    s += -(u00 + u10) * y0[zl];
+    s += -u10 * y0[zl + xh];
+    s += -(u00 + u01) * c[zl + xl];
+    s += -(u10 + u11) * c[zl + xh];
+    s += -u01 * y2[zl + xl];
+    s += -(u01 + u11) * y2[zl];
+    s += -u11 * y2[zl + xh];
+    s += -(u00 + v00) * y0[xl];
+    s += -(u10 + v10) * y0[xh];
+    s += -(u01 + v01) * y2[xl];
+    s += -(u11 + v11) * y2[xh];
+    s += -v00 * y0[zh + xl];
+    s += -(v00 + v10) * y0[zh];
+    s += -v10 * y0[zh + xh];
+    s += -(v00 + v01) * c[zh + xl];
+    s += -(v10 + v11) * c[zh + xh];
+    s += -v01 * y2[zh + xl];
+    s += -(v01 + v11) * y2[zh];
+    s += -v11 * y2[zh + xh];
+    T c8 = 0;
+    c8 += u00;
+    c8 += u10;
+    c8 += u01;
+    c8 += u11;
+    c8 += v00;
+    c8 += v10;
+    c8 += v01;
+    c8 += v11;
+    diag = (T)4 * c8;
     return s;
 }
 

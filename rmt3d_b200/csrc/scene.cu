@@ -943,8 +943,18 @@ constexpr int kDiagVals = 8;
 
 __global__ void k_mean(const double *x, size_t n, double scale, double *out, unsigned *ticket) {
     double sum = 0;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        sum += x[i] * scale;
+    // eight loads in flight, added in order (one load at a time took 75 us on
+    // 193^3 nodes, whose DRAM time is 9 us)
+    const size_t ts = (size_t)gridDim.x * blockDim.x;
+    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    for (; i + 7 * ts < n; i += 8 * ts) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[q] = x[i + q * ts];
+#pragma unroll
+        for (int q = 0; q < 8; q++) sum += v[q] * scale;
+    }
+    for (; i < n; i += ts) sum += x[i] * scale;
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     __shared__ double sh[32];
     __shared__ bool last;

@@ -1,6 +1,7 @@
 // Runs the device code of the shared-memory V-cycle (mg_slab.cuh) on host
 // threads -- one per CUDA thread, a cluster of small CTAs -- and compares it
-// bit for bit with the per-phase V-cycle of mg_ops.cuh.  Built with the
+// bit for bit with the per-phase V-cycle of mg_ops.cuh, and that operator with
+// its term-by-term form (ref_ops.inc).  Built with the
 // address sanitizer, every CTA's shared memory a heap block of its own size,
 // so an index outside it ends the run.
 //   slab_sim kind(0 MAC, 1 FEM) vd f64 n0 n1 n2 p0 p1 p2 csize v_down v_up l0 seed
@@ -95,7 +96,30 @@ int fail(int code, const std::string &) { return code; }
 }  // namespace rmt3d
 #include "mg_slab.cuh"
 
+namespace rmt3d {
+#include "ref_ops.inc"
+}
 using namespace rmt3d;
+
+// one row of the operator, as the kernels form it and term by term: the same
+// updated value and residual
+template <typename T, int KIND, bool VD>
+static size_t check_rows(const pmg_level &P, T rv) {
+    const lvl_dev L = ldev(P);
+    const T *x = LX<T>(P), *ri = VD ? LRI<T>(P) : nullptr;
+    size_t bad = 0;
+    for (int k = 0; k < L.n2; k++)
+        for (int j = 0; j < L.n1; j++)
+            for (int i = 0; i < L.n0; i++) {
+                T d1, d2;
+                const T s1 = op_offdiag<T>(KIND, L, x, ri, i, j, k, d1);
+                const T s2 = KIND ? (VD ? ref_fem_offdiag_vd(L, x, ri, i, j, k, d2) : ref_fem_offdiag(L, x, i, j, k, d2))
+                                  : (VD ? ref_mac_offdiag_vd(L, x, ri, i, j, k, d2) : ref_mac_offdiag(L, x, i, j, k, d2));
+                const T a = (rv - s1) / d1, b = (rv - s2) / d2;
+                if (memcmp(&a, &b, sizeof(T)) || memcmp(&d1, &d2, sizeof(T)) || s1 != s2) bad++;
+            }
+    return bad;
+}
 
 static int plan(int kind, const int n[3], const int prd[3], std::vector<mg_level> &lv) {
     mg_level L;
@@ -148,6 +172,15 @@ static int run(const std::vector<mg_level> &lv, int csize, int vdn, int vup, int
         for (int d = 0; d < 3; d++) A.lv[l].n[d] = lv[l].n[d], A.lv[l].prd[d] = lv[l].prd[d];
         set_level_ptrs<T>(A.lv[l], x[l].data(), r[l].data(), s[l].data());
         if (VD) (sizeof(T) == 8 ? (void)(A.lv[l].ri = (double *)ri[l].data()) : (void)(A.lv[l].ris = (float *)ri[l].data()));
+    }
+    for (int l = 0; l < A.nlev; l++) {
+        const std::vector<T> keep_x = x[l];
+        for (auto &v : x[l]) v = (T)U(rng);
+        if (size_t bad = check_rows<T, KIND, VD>(A.lv[l], (T)0.37)) {
+            printf("level %d: %zu rows differ from the term-by-term operator\n", l, bad);
+            return 5;
+        }
+        x[l] = keep_x;
     }
     const std::vector<T> x0 = x[l0];
     slab_args S;
