@@ -183,19 +183,6 @@ __device__ inline void join_layer(int c, uint8_t *lay, int *inl, int next, int *
     if (atomicCAS(inl + c, 0, next) == 0) front[list_slot(cnt)] = c;
 }
 
-// the free orthogonal neighbours of cell ind join layer `next`
-__device__ inline void push_from(const grid_dev &g, int ind, uint8_t *lay, int *inl, int next, int *front,
-                                 int *cnt) {
-    const int strides[3] = {1, g.sm4, g.smn4};
-    int k = ind / g.smn4, j = (ind % g.smn4) / g.sm4, i = ind % g.sm4;
-    if (!inner_ghost(g, i, j, k)) return;
-    for (int d = 0; d < 3; d++)
-        for (int sg = -1; sg <= 1; sg += 2) {
-            int c = ind + sg * strides[d];
-            if (lay[c] == 255) join_layer(c, lay, inl, next, front, cnt);
-        }
-}
-
 // (object, index) of entry t of the concatenated frontiers; false past the end
 __device__ inline bool front_entry(int n_obj, const int *cnt, int &t, int &o) {
     for (o = 0; o < n_obj; o++) {
@@ -205,28 +192,45 @@ __device__ inline bool front_entry(int n_obj, const int *cnt, int &t, int &o) {
     return false;
 }
 
-// neighbours of the primary cells (from_primary) or of the current
-// frontiers (front, cnt) join the next layer, listed in nfront / ncnt
-// (add_to_next_list with the orthogonal rule, extrap_helper.hh:166-255)
-__global__ void k_lay_push(grid_dev g, const int *front, const int *cnt, int from_primary, uint8_t *lay, int *inl,
-                           int next, int *nfront, int *ncnt) {
-    if (from_primary) {
-        int ind = blockIdx.x * blockDim.x + threadIdx.x;
-        if (ind >= g.ncell) return;
-        for (int o = 0; o < g.n_obj; o++) {
-            const size_t off = (size_t)o * g.ncell;
-            if (lay[off + ind] == 0) push_from(g, ind, lay + off, inl + off, next, nfront + off, ncnt + o);
-        }
-        return;
+// the free orthogonal neighbours of the primary cells join layer 1
+// (add_to_next_list with the orthogonal rule, extrap_helper.hh:166-255); a
+// cell's six tags are loaded together
+__global__ void k_lay_push(grid_dev g, uint8_t *lay, int *inl, int *nfront, int *ncnt) {
+    const int ind = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ind >= g.ncell) return;
+    const int k = ind / g.smn4, j = (ind / g.sm4) % g.sn4, i = ind % g.sm4;
+    if (!inner_ghost(g, i, j, k)) return;
+    const int nb[6] = {ind - 1, ind + 1, ind - g.sm4, ind + g.sm4, ind - g.smn4, ind + g.smn4};
+    for (int o = 0; o < g.n_obj; o++) {
+        const size_t off = (size_t)o * g.ncell;
+        if (lay[off + ind] != 0) continue;
+        bool free_[6];
+#pragma unroll
+        for (int d = 0; d < 6; d++) free_[d] = lay[off + nb[d]] == 255;
+#pragma unroll
+        for (int d = 0; d < 6; d++)
+            if (free_[d]) join_layer(nb[d], lay + off, inl + off, 1, nfront + off, ncnt + o);
     }
+}
+
+// The same from the listed cells of a layer to the next one, one thread per
+// (cell, neighbour): tag, claim and append are a chain of memory latencies,
+// and one thread walking its six neighbours made it six times as long (7.6 us
+// a layer; the pass now hides behind the layer's fits, whose launch it shares).
+__device__ inline void push_layer(const grid_dev &g, const int *front, const int *cnt, uint8_t *lay, int *inl, int next,
+                                  int *nfront, int *ncnt, int t0, int ts) {
     int total = 0;
     for (int o = 0; o < g.n_obj; o++) total += cnt[o];
-    if (blockIdx.x * blockDim.x >= total) return;  // no frontier entry in any round
-    for (int t0 = blockIdx.x * blockDim.x + threadIdx.x; t0 < total; t0 += gridDim.x * blockDim.x) {
-        int t = t0, o;
+    for (int q = t0; q < 6 * total; q += ts) {
+        int t = q / 6, o;
+        const int d = q - 6 * t;
         if (!front_entry(g.n_obj, cnt, t, o)) break;
         const size_t off = (size_t)o * g.ncell;
-        push_from(g, front[off + t], lay + off, inl + off, next, nfront + off, ncnt + o);
+        const int ind = front[off + t];
+        const int k = ind / g.smn4, j = (ind / g.sm4) % g.sn4, i = ind % g.sm4;
+        if (!inner_ghost(g, i, j, k)) continue;
+        const int st = d < 2 ? 1 : (d < 4 ? g.sm4 : g.smn4), c = (d & 1) ? ind + st : ind - st;
+        if (lay[off + c] == 255) join_layer(c, lay + off, inl + off, next, nfront + off, ncnt + o);
     }
 }
 
@@ -270,12 +274,64 @@ __device__ inline double group_sum(double v, unsigned mask) {
     return v;
 }
 
+// The warp's sums of N values, in every lane: halves of the values change
+// sides at each step, so the sums cost N + 1 exchanges and N broadcasts
+// instead of 5 N exchanges.  Every sum pairs the lanes as group_sum<32> does
+// (a + b == b + a): the same bits.
+template <int N>
+__device__ inline void warp_sums(double (&v)[N]) {
+    static_assert(N == 8 || N == 16, "8 or 16 values");
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h /= 2) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int q = 0; q < h; q++) {
+            const double send = up ? v[q] : v[q + h], kept = up ? v[q + h] : v[q];
+            v[q] = kept + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+        o >>= 1;
+    }
+    double mine = v[0];
+    for (; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+#pragma unroll
+    for (int q = 0; q < N; q++) v[q] = __shfl_sync(0xffffffffu, mine, q * (32 / N));
+}
+
 // -------------------------------------------------------------------------
 // One layer of least-squares extrapolation, one lane group per frontier cell:
 // gather_and_list (fluid_3d_ex.cc:86-272), extrap_helper::least_square
 // (extrap_helper.cc:34-103) with lin_sys (:129-146), mat3::inverse
 // (Utilities/mat3.hh:61-67) and transfer (fluid_3d_ex.cc:293-328).
 // -------------------------------------------------------------------------
+// the fit from its weighted normal equations about the averages: false when
+// they are singular
+__device__ inline bool ls_solve(const double (&a)[6], const double (&rhs)[9], const double (&davg)[3],
+                                const double (&ravg)[3], double cx, double cy, double cz, double (&val)[3]) {
+    // mat3 A(XX, XY, XZ, XY, YY, YZ, XZ, YZ, ZZ) and its inverse
+    const double a11 = a[0], a12 = a[3], a13 = a[4], a21 = a[3], a22 = a[1], a23 = a[5], a31 = a[4],
+                 a32 = a[5], a33 = a[2];
+    double det = a11 * (a22 * a33 - a23 * a32) + a21 * (a13 * a32 - a12 * a33) + a31 * (a12 * a23 - a13 * a22);
+    if (fabs(det) < 1e-17) return false;
+    double id = 1 / det;
+    double inv[9] = {(a22 * a33 - a23 * a32) * id, (a13 * a32 - a12 * a33) * id, (a12 * a23 - a13 * a22) * id,
+                     (a23 * a31 - a21 * a33) * id, (a11 * a33 - a13 * a31) * id, (a13 * a21 - a11 * a23) * id,
+                     (a21 * a32 - a22 * a31) * id, (a12 * a31 - a11 * a32) * id, (a11 * a22 - a12 * a21) * id};
+    double ps[3] = {cx - davg[0], cy - davg[1], cz - davg[2]};
+    for (int c = 0; c < 3; c++) {
+        double co0 = inv[0] * rhs[3 * c] + inv[1] * rhs[3 * c + 1] + inv[2] * rhs[3 * c + 2];
+        double co1 = inv[3] * rhs[3 * c] + inv[4] * rhs[3 * c + 1] + inv[5] * rhs[3 * c + 2];
+        double co2 = inv[6] * rhs[3 * c] + inv[7] * rhs[3 * c + 1] + inv[8] * rhs[3 * c + 2];
+        double v = ravg[c];
+        v += co0 * ps[0];
+        v += co1 * ps[1];
+        v += co2 * ps[2];
+        val[c] = v;
+    }
+    return true;
+}
+
 constexpr int kPowTab = 64;
 
 // One radius R of the least-squares fit for the frontier cell (ii, jj, kk)
@@ -381,49 +437,123 @@ __device__ bool ls_radius(const grid_dev &g, const objmap_dev &m, int R, int L, 
     }
     for (int c = 0; c < 6; c++) a[c] = group_sum<LANES>(a[c], gm);
     for (int c = 0; c < 9; c++) rhs[c] = group_sum<LANES>(rhs[c], gm);
-    // mat3 A(XX, XY, XZ, XY, YY, YZ, XZ, YZ, ZZ) and its inverse
-    const double a11 = a[0], a12 = a[3], a13 = a[4], a21 = a[3], a22 = a[1], a23 = a[5], a31 = a[4],
-                 a32 = a[5], a33 = a[2];
-    double det = a11 * (a22 * a33 - a23 * a32) + a21 * (a13 * a32 - a12 * a33) + a31 * (a12 * a23 - a13 * a22);
-    if (fabs(det) < 1e-17) return false;
-    double id = 1 / det;
-    double inv[9] = {(a22 * a33 - a23 * a32) * id, (a13 * a32 - a12 * a33) * id, (a12 * a23 - a13 * a22) * id,
-                     (a23 * a31 - a21 * a33) * id, (a11 * a33 - a13 * a31) * id, (a13 * a21 - a11 * a23) * id,
-                     (a21 * a32 - a22 * a31) * id, (a12 * a31 - a11 * a32) * id, (a11 * a22 - a12 * a21) * id};
-    double ps[3] = {cx - davg[0], cy - davg[1], cz - davg[2]};
-    for (int c = 0; c < 3; c++) {
-        double co0 = inv[0] * rhs[3 * c] + inv[1] * rhs[3 * c + 1] + inv[2] * rhs[3 * c + 2];
-        double co1 = inv[3] * rhs[3 * c] + inv[4] * rhs[3 * c + 1] + inv[5] * rhs[3 * c + 2];
-        double co2 = inv[6] * rhs[3 * c] + inv[7] * rhs[3 * c + 1] + inv[8] * rhs[3 * c + 2];
-        double v = ravg[c];
-        v += co0 * ps[0];
-        v += co1 * ps[1];
-        v += co2 * ps[2];
-        val[c] = v;
+    return ls_solve(a, rhs, davg, ravg, cx, cy, cz, val);
+}
+
+// The first radius (2: 5^3 candidates) with a warp per cell: the candidates'
+// codes and values, four a lane, come in `cd` and `xv`, loaded at once before
+// the cell's normal was formed, and stay in registers with their weights for
+// the second pass.  The loop form above loads them again for it, one round of
+// loads after another, and sums with 5 exchanges a value: 20 us a layer of a
+// 64^3 sphere scene, 54 us of a 96^3 scene with five; this form 15 and 41 us,
+// the next layer's listing included.  It is a chain of dependent loads and FP64
+// divisions, not bandwidth.  Operations and their order are those of
+// ls_radius<5, 32>.
+__device__ inline bool ls_first(const int (&cd)[4], const double (&xv)[4][3], int L, int lane, int ii, int jj, int kk,
+                                bool directional, const double (&gph)[3], double cx, double cy, double cz,
+                                const double *lx, const double *ly, const double *lz, const double *wpow,
+                                double (&val)[3]) {
+    double wg[4], d[4][3], acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    bool use[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        use[u] = cd[u] >= 0 && cd[u] < L;
+        if (!use[u]) continue;
+        const int s = lane + 32 * u, p = s % 5 - 2, q = (s / 5) % 5 - 2, r = s / 25 - 2;
+        d[u][0] = lx[ii + p], d[u][1] = ly[jj + q], d[u][2] = lz[kk + r];
+        double wgt = wpow[abs(p) + abs(q) + abs(r)];
+        if (directional) {
+            const double ev[3] = {cx - d[u][0], cy - d[u][1], cz - d[u][2]};
+            double dw = 0, en = 0;
+            for (int pp = 0; pp < 3; pp++) {
+                dw += ev[pp] * gph[pp];
+                en += ev[pp] * ev[pp];
+            }
+            en = sqrt(en);
+            dw /= en;
+            dw *= wgt;
+            if (!(dw > 0)) {
+                use[u] = false;
+                continue;
+            }
+            wgt = dw;
+        }
+        wg[u] = wgt;
+        acc[0] += wgt;
+        acc[7] += 1;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            acc[1 + c] += d[u][c] * wgt;
+            acc[4 + c] += xv[u][c] * wgt;
+        }
     }
-    return true;
+    warp_sums<8>(acc);
+    if (acc[7] == 0) return false;
+    double davg[3], ravg[3];
+    for (int c = 0; c < 3; c++) {
+        ravg[c] = acc[4 + c] / acc[0];
+        davg[c] = acc[1 + c] / acc[0];
+    }
+    double m2[16];
+#pragma unroll
+    for (int c = 0; c < 16; c++) m2[c] = 0;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        if (!use[u]) continue;
+        const double Q = wg[u];
+        const double e0 = d[u][0] - davg[0], e1 = d[u][1] - davg[1], e2 = d[u][2] - davg[2];
+        m2[0] += Q * e0 * e0;
+        m2[1] += Q * e1 * e1;
+        m2[2] += Q * e2 * e2;
+        m2[3] += Q * e0 * e1;
+        m2[4] += Q * e0 * e2;
+        m2[5] += Q * e1 * e2;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const double lr = Q * (xv[u][c] - ravg[c]);
+            m2[6 + 3 * c + 0] += e0 * lr;
+            m2[6 + 3 * c + 1] += e1 * lr;
+            m2[6 + 3 * c + 2] += e2 * lr;
+        }
+    }
+    warp_sums<16>(m2);
+    double a[6], rhs[9];
+#pragma unroll
+    for (int c = 0; c < 6; c++) a[c] = m2[c];
+#pragma unroll
+    for (int c = 0; c < 9; c++) rhs[c] = m2[6 + c];
+    return ls_solve(a, rhs, davg, ravg, cx, cy, cz, val);
 }
 
 // Every object's frontier in one launch: lane group w (LANES lanes)
 // takes entry w of the concatenated frontiers.  The weights wt^n (n = |p|+|q|+|r|) come from a
 // per-block table of the same pow() values.
+// The first npush blocks list the next layer's cells instead (push_layer;
+// next 0: none): they read the same lists and write what no fit reads.
 template <int LANES>
-__global__ void k_extrap_layer(grid_dev g, const fields_dev *__restrict__ F, const int *front, const int *cnt, int L,
-                               int max_rs, double wt, const double *lx, const double *ly, const double *lz,
-                               int *err) {
+__global__ void __launch_bounds__(128) k_extrap_layer(grid_dev g, const fields_dev *__restrict__ F, const int *front,
+                                                      const int *cnt, int L, int max_rs, double wt, const double *lx,
+                                                      const double *ly, const double *lz, int *err, int npush,
+                                                      uint8_t *lay, int *inl, int next, int *nfront, int *ncnt) {
+    if ((int)blockIdx.x < npush) {
+        push_layer(g, front, cnt, lay, inl, next, nfront, ncnt, blockIdx.x * blockDim.x + threadIdx.x,
+                   npush * blockDim.x);
+        return;
+    }
     __shared__ double wpow[kPowTab];
+    const int blk = (int)blockIdx.x - npush, nblk = (int)gridDim.x - npush;
     int total = 0;
     for (int o = 0; o < g.n_obj; o++) total += cnt[o];
     // the grid is sized for the largest frontiers: a block whose first lane
     // group is past this layer's frontier has no cell in any round and leaves
     // before building its weight table (the whole block, so no barrier waits)
-    if (blockIdx.x * (blockDim.x / LANES) >= total) return;
+    if (blk * (int)(blockDim.x / LANES) >= total) return;
     const int npow = 3 * max_rs + 1;
     for (int q = threadIdx.x; q < kPowTab && q < npow; q += blockDim.x) wpow[q] = pow(wt, (double)q);
     __syncthreads();
     const int lane = threadIdx.x & (LANES - 1);
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / LANES;
-    const int nwarps = (gridDim.x * blockDim.x) / LANES;
+    const int warp = (blk * blockDim.x + threadIdx.x) / LANES;
+    const int nwarps = (nblk * blockDim.x) / LANES;
     for (int t0 = warp; t0 < total; t0 += nwarps) {
         int t = t0, o;
         if (!front_entry(g.n_obj, cnt, t, o)) break;
@@ -431,10 +561,25 @@ __global__ void k_extrap_layer(grid_dev g, const fields_dev *__restrict__ F, con
         const int ind = front[(size_t)o * g.ncell + t];
         const int kk = ind / g.smn4, jj = (ind % g.smn4) / g.sm4, ii = ind % g.sm4;
         if (image_backed(g, ii, jj, kk)) continue;  // within_extrapolation_domain
+        int cd[4];
+        double xv[4][3];
+        if (LANES == 32) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int s = lane + 32 * u, p = s % 5 - 2, q = (s / 5) % 5 - 2, r = s / 25 - 2;
+                const bool in = s < 125 && ii + p >= 0 && ii + p < g.sm4 && jj + q >= 0 && jj + q < g.sn4 &&
+                                kk + r >= 0 && kk + r < g.so4;
+                const int qi = in ? ind + p + g.sm4 * q + g.smn4 * r : ind;
+                cd[u] = in ? m.code[qi] : -1;
+#pragma unroll
+                for (int c = 0; c < 3; c++) xv[u][c] = m.xp[c][qi];
+            }
+        }
         // average of the previous step's interface normals over the six faces
         double gph[3] = {0, 0, 0};
         double gnorm = 0;
-        if (ii >= 2 && ii <= g.sm4 - 3 && jj >= 2 && jj <= g.sn4 - 3 && kk >= 2 && kk <= g.so4 - 3) {
+        // (only the first two layers weight by direction)
+        if (L <= 2 && ii >= 2 && ii <= g.sm4 - 3 && jj >= 2 && jj <= g.sn4 - 3 && kk >= 2 && kk <= g.so4 - 3) {
             const int pidx[4] = {ind, ind + 1, ind + g.sm4, ind + g.smn4};
             int nfaces = 0;
             for (int pp = 0; pp < 4; pp++) {
@@ -475,7 +620,12 @@ __global__ void k_extrap_layer(grid_dev g, const fields_dev *__restrict__ F, con
         const double cx = lx[ii], cy = ly[jj], cz = lz[kk];
         bool success = false;
         double val[3] = {0, 0, 0};
-        for (int R = 2; R <= max_rs && !success; R++) {
+        int R = 2;
+        if (LANES == 32 && max_rs >= 2) {
+            success = ls_first(cd, xv, L, lane, ii, jj, kk, directional, gph, cx, cy, cz, lx, ly, lz, wpow, val);
+            R = 3;
+        }
+        for (; R <= max_rs && !success; R++) {
 #define LS_ARGS g, m, R, L, lane, ii, jj, kk, ind, directional, gph, cx, cy, cz, lx, ly, lz, wpow, wt, val
             switch (R) {
                 case 2: success = ls_radius<5, LANES>(LS_ARGS); break;
@@ -501,9 +651,11 @@ __global__ void k_extrap_layer(grid_dev g, const fields_dev *__restrict__ F, con
 }
 
 template __global__ void k_extrap_layer<4>(grid_dev, const fields_dev *__restrict__, const int *, const int *, int,
-                                            int, double, const double *, const double *, const double *, int *);
+                                            int, double, const double *, const double *, const double *, int *, int,
+                                            uint8_t *, int *, int, int *, int *);
 template __global__ void k_extrap_layer<32>(grid_dev, const fields_dev *__restrict__, const int *, const int *, int,
-                                             int, double, const double *, const double *, const double *, int *);
+                                             int, double, const double *, const double *, const double *, int *, int,
+                                             uint8_t *, int *, int, int *, int *);
 
 // communicate_a_layer on one rank (fluid_3d_comm.cc:203-280): image-backed
 // ghosts receive the maps of the layer just made at their image (periodic

@@ -141,7 +141,7 @@ struct rmt3d_scene {
     uint8_t *lay = nullptr;  // per object: layer tags
     int *inl = nullptr;      // per object: layer that claimed the cell (0: none)
     int *front[2] = {nullptr, nullptr};  // per object: ncell entries each
-    int *fcnt = nullptr;                  // frontier lengths, [2][kMaxObj]
+    int *fcnt = nullptr;                  // frontier lengths, [nlayers][kMaxObj]
     // lanes per frontier cell of the least-squares extrapolation: a warp when
     // the scene steps on its own, 4 when it steps inside a group with others
     int extrap_lanes = 32;
@@ -407,40 +407,39 @@ static void extrapolate(rmt3d_scene *s, bool lay_ready = false) {
     // without a periodic axis no ghost cell is the image of an interior
     // cell, and the two ghost-copy kernels would find nothing to do
     const bool prd = g.prd[0] || g.prd[1] || g.prd[2];
-    int *cnt[2] = {s->fcnt, s->fcnt + kMaxObj};
+    // a list length per layer, all zeroed at once
+    auto cnt = [&](int layer) { return s->fcnt + (layer - 1) * kMaxObj; };
     if (!lay_ready) {
         k_lay_init<<<nb, 256, 0, s->st>>>(g, s->dF, s->lay, s->inl);
         s->count();
     }
-    cudaMemsetAsync(s->fcnt, 0, 2 * kMaxObj * sizeof(int), s->st);
-    k_lay_push<<<nb, 256, 0, s->st>>>(g, nullptr, nullptr, 1, s->lay, s->inl, 1, s->front[0], cnt[0]);
+    cudaMemsetAsync(s->fcnt, 0, s->d.nlayers * kMaxObj * sizeof(int), s->st);
+    k_lay_push<<<nb, 256, 0, s->st>>>(g, s->lay, s->inl, s->front[0], cnt(1));
     s->count();
     if (prd) {
-        k_lay_ghost<<<nb, 256, 0, s->st>>>(g, s->lay, s->inl, 1, s->front[0], cnt[0]);
+        k_lay_ghost<<<nb, 256, 0, s->st>>>(g, s->lay, s->inl, 1, s->front[0], cnt(1));
         s->count();
     }
     int cur = 0;
     for (int L = 1; L <= s->d.nlayers; L++) {
+        // the layer's fits and, beside them, the next layer's list
+        const bool more = L < s->d.nlayers;
+        const int npush = more ? 148 : 0;
         auto kern = s->extrap_lanes == 4 ? k_extrap_layer<4> : k_extrap_layer<32>;
-        kern<<<per_warp_blocks, 128, 0, s->st>>>(g, s->dF, s->front[cur], cnt[cur], L, s->d.max_extrap_rs,
-                                                 s->d.weight_fac, s->lx, s->ly, s->lz, s->counters + 2);
+        kern<<<npush + per_warp_blocks, 128, 0, s->st>>>(g, s->dF, s->front[cur], cnt(L), L, s->d.max_extrap_rs,
+                                                         s->d.weight_fac, s->lx, s->ly, s->lz, s->counters + 2, npush,
+                                                         s->lay, s->inl, L + 1, s->front[cur ^ 1],
+                                                         more ? cnt(L + 1) : nullptr);
         s->count();
         if (prd) {
             k_layer_ghost_copy<<<nb, 256, 0, s->st>>>(g, s->dF, L);
             s->count();
         }
-        if (L < s->d.nlayers) {
-            int nxt = cur ^ 1;
-            cudaMemsetAsync(cnt[nxt], 0, kMaxObj * sizeof(int), s->st);
-            k_lay_push<<<per_warp_blocks, 256, 0, s->st>>>(g, s->front[cur], cnt[cur], 0, s->lay, s->inl, L + 1,
-                                                           s->front[nxt], cnt[nxt]);
+        if (more && prd) {
+            k_lay_ghost<<<nb, 256, 0, s->st>>>(g, s->lay, s->inl, L + 1, s->front[cur ^ 1], cnt(L + 1));
             s->count();
-            if (prd) {
-                k_lay_ghost<<<nb, 256, 0, s->st>>>(g, s->lay, s->inl, L + 1, s->front[nxt], cnt[nxt]);
-                s->count();
-            }
-            cur = nxt;
         }
+        cur ^= 1;
     }
 }
 
@@ -1950,7 +1949,7 @@ extern "C" int rmt3d_scene_create(const rmt3d_scene_desc *desc, void *stream, rm
     if (d.n_obj > 0) {
         const size_t no = (size_t)d.n_obj * n;
         s->plan(&s->lay, no), s->plan(&s->inl, no), s->plan(&s->front[0], no), s->plan(&s->front[1], no);
-        s->plan(&s->fcnt, 2 * kMaxObj), s->plan(&s->mlist, n), s->plan(&s->mcnt, 1);
+        s->plan(&s->fcnt, (size_t)d.nlayers * kMaxObj), s->plan(&s->mlist, n), s->plan(&s->mcnt, 1);
     }
     e |= s->commit_slab();
     for (int o = 0; o < d.n_obj && !e; o++) {
@@ -2925,7 +2924,7 @@ extern "C" size_t rmt3d_scene_footprint(const rmt3d_scene_desc *d) {
     b += (size_t)d->n_obj * (2 * slab_pad(n * sizeof(int)) + 51 * slab_pad(n * sizeof(double)));
     if (d->n_obj > 0) {
         const size_t no = (size_t)d->n_obj * n;
-        b += slab_pad(no * sizeof(uint8_t)) + 3 * slab_pad(no * sizeof(int)) + slab_pad(2 * kMaxObj * sizeof(int)) +
+        b += slab_pad(no * sizeof(uint8_t)) + 3 * slab_pad(no * sizeof(int)) + slab_pad((size_t)d->nlayers * kMaxObj * sizeof(int)) +
              slab_pad(n * sizeof(int)) + slab_pad(sizeof(int));
     }
     if ((d->run.dump_code & 1) && d->run.ntracers > 0)
