@@ -151,9 +151,12 @@ struct fields_dev {
     float *fvel32[18];    // face states in FP32 (RMT3D_MIXED_BULK32 only)
     double *sigma[9];
     double *rho;  // VAR_DEN density per cell (fluid_3d.hh:160)
-    objmap_dev om[kMaxObj];
-    unsigned int *flags;  // scratch per-cell flags (extrapolation frontier)
+    int *code[kMaxObj];    // the objects' map codes (om[o].code)
+    const objmap_dev *om;  // the objects' map arrays, a table in device memory
 };
+// The step's kernels take this by value (0.6 KB of launch parameters), so an
+// array's address is a constant-bank read; fetched through a pointer it was a
+// load of its own before every load of data.
 
 // Velocity face states fvel[f][c] (fields.hh:296), written by the edge
 // extrapolation and read by the upwinding, both projections and the momentum
@@ -191,7 +194,7 @@ __device__ inline unsigned map_mask(const grid_dev &g, const fields_dev *__restr
     for (int base = 0; base < g.n_obj; base += 4) {
         int c[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) c[u] = base + u < g.n_obj ? F->om[base + u].code[ind] : -1;
+        for (int u = 0; u < 4; u++) c[u] = base + u < g.n_obj ? F->code[base + u][ind] : -1;
 #pragma unroll
         for (int u = 0; u < 4; u++)
             if (c[u] >= 0) m |= 1u << (base + u);

@@ -10,7 +10,9 @@ namespace rmt3d {
 // shuffles, then the warps of a block in index order, then (in the block
 // that finishes last) the blocks in index order.  Bit c of max_mask makes
 // value c a maximum instead of a sum.  out holds NV totals followed by NV
-// partials per block; *ticket returns to 0.  blockDim.x is a multiple of 32.
+// partials per block; *ticket returns to 0.  blockDim.x is a multiple of 32,
+// gridDim.x at most kRedBlocks.
+constexpr int kRedBlocks = 148;
 template <int NV>
 __device__ void fixed_order_reduce(double (&v)[NV], unsigned max_mask, double *out, unsigned *ticket) {
     __shared__ double sh[NV][32];
@@ -36,12 +38,19 @@ __device__ void fixed_order_reduce(double (&v)[NV], unsigned max_mask, double *o
         last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
     }
     __syncthreads();
-    if (last && threadIdx.x < NV) {
-        __threadfence();
+    if (!last) return;
+    // the whole block fetches the partials, one thread a value adds them in
+    // block order (fetching them one by one as well was a chain of 148 L2
+    // latencies)
+    __shared__ double part[NV * kRedBlocks];
+    __threadfence();
+    for (int t = threadIdx.x; t < NV * (int)gridDim.x; t += blockDim.x) part[t] = __ldcg(out + NV + t);
+    __syncthreads();
+    if (threadIdx.x < NV) {
         const int c = threadIdx.x;
         const bool mx = (max_mask >> c) & 1u;
-        const volatile double *part = out + NV;
         double a = part[c];
+#pragma unroll 4
         for (unsigned b = 1; b < gridDim.x; b++) a = mx ? fmax(a, part[NV * b + c]) : a + part[NV * b + c];
         out[c] = a;
         if (c == 0) *ticket = 0;

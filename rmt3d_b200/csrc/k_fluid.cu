@@ -90,7 +90,8 @@ __global__ void k_bc_cc(grid_dev g, int n, bc_face lo, bc_face hi, double *u, do
 // All wall faces in one launch (blockIdx.z = face; bit f of walls marks a
 // wall): each face reads velocities only and writes its own face-velocity
 // components, so the faces are independent.
-__global__ void k_bc_cf(grid_dev g, int walls, bc_faces bcs, const fields_dev *F) {
+__global__ void k_bc_cf(grid_dev g, int walls, bc_faces bcs, const __grid_constant__ fields_dev F_) {
+    const fields_dev *__restrict__ F = &F_;
     const int face = blockIdx.z;
     if (!((walls >> face) & 1)) return;
     const bc_face &bc = bcs.f[face];
@@ -237,12 +238,12 @@ __device__ void face_stress(const grid_dev &g, const fields_dev *__restrict__ F,
     int order[kMaxObj];
     int nmaps = 0, prim = -1;
     for (int o = 0; o < g.n_obj; o++) {
-        int cd = F->om[o].code[ind];
+        int cd = F->code[o][ind];
         if (cd == 0) prim = o;
     }
     if (prim >= 0) order[nmaps++] = prim;
     for (int o = 0; o < g.n_obj; o++)
-        if (o != prim && F->om[o].code[ind] > 0) order[nmaps++] = o;
+        if (o != prim && F->code[o][ind] > 0) order[nmaps++] = o;
 
     for (int mi = 0; mi < nmaps; mi++) {
         const int o = order[mi];
@@ -364,8 +365,9 @@ __device__ void face_stress(const grid_dev &g, const fields_dev *__restrict__ F,
 // disjoint outputs and read only what no face writes, so they run in any
 // order; a thread holds one face's state instead of three, and every lane of
 // a warp has a map cell to work on.
-__global__ void __launch_bounds__(128) k_stress(grid_dev g, const fields_dev *__restrict__ F, const int *list,
+__global__ void __launch_bounds__(128) k_stress(grid_dev g, const __grid_constant__ fields_dev F_, const int *list,
                                                 const int *cnt) {
+    const fields_dev *__restrict__ F = &F_;
     const int n = *cnt;
     const long total = 3L * n;
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
@@ -385,7 +387,8 @@ __global__ void __launch_bounds__(128) k_stress(grid_dev g, const fields_dev *__
 // sfrac = ss = 0), in a small kernel that keeps many more threads resident
 // than the full one.  Cells that hold any map are appended to list (when
 // given) for the full stress kernel, one atomic per warp.
-__global__ void k_stress_fluid(grid_dev g, const fields_dev *__restrict__ F, int *list, int *cnt) {
+__global__ void k_stress_fluid(grid_dev g, const __grid_constant__ fields_dev F_, int *list, int *cnt) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -527,8 +530,8 @@ __device__ void acceleration(const grid_dev &g, const fields_dev *__restrict__ F
     double sfrac = 0;
     const double xx = lx[i], yy = ly[j], zz = lz[k];
     for (int o = 0; o < g.n_obj; o++) {
+        if (F->code[o][ind] < 0) continue;
         const objmap_dev &m = F->om[o];
-        if (m.code[ind] < 0) continue;
         double rv[3] = {m.x[0][ind], m.x[1][ind], m.x[2][ind]};
         double phiv = obj_phi(g, o, rv[0], rv[1], rv[2]);
         if (phiv < g.eps) {
@@ -594,9 +597,10 @@ __device__ __forceinline__ void edge_store_f32(const grid_dev &g, const fields_d
 // (fields.hh:147-177, non-TANG branch).  Interior cells.
 // -------------------------------------------------------------------------
 template <typename FT>
-__global__ void __launch_bounds__(256, 3) k_edge_vel(grid_dev g, const fields_dev *__restrict__ F, const double *lx,
+__global__ void __launch_bounds__(256, 3) k_edge_vel(grid_dev g, const __grid_constant__ fields_dev F_, const double *lx,
                                                      const double *ly, const double *lz, double cdt,
                                                      const double *time_p, int var_den) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
     int k = blockIdx.z * blockDim.z + threadIdx.z + 2;
@@ -637,9 +641,9 @@ __global__ void __launch_bounds__(256, 3) k_edge_vel(grid_dev g, const fields_de
         edge_store_f32(g, F, ind, vel, nv, acc, cdt);
     }
 }
-template __global__ void k_edge_vel<double>(grid_dev, const fields_dev *__restrict__, const double *, const double *,
+template __global__ void k_edge_vel<double>(grid_dev, const __grid_constant__ fields_dev, const double *, const double *,
                                             const double *, double, const double *, int);
-template __global__ void k_edge_vel<float>(grid_dev, const fields_dev *__restrict__, const double *, const double *,
+template __global__ void k_edge_vel<float>(grid_dev, const __grid_constant__ fields_dev, const double *, const double *,
                                            const double *, double, const double *, int);
 
 // -------------------------------------------------------------------------
@@ -694,12 +698,13 @@ __device__ __forceinline__ bool ev_wait(uint64_t *bar, unsigned parity) {
 }
 
 template <typename FT>
-__global__ void __launch_bounds__(256, 2) k_edge_vel_tma(grid_dev g, const fields_dev *__restrict__ F,
+__global__ void __launch_bounds__(256, 2) k_edge_vel_tma(grid_dev g, const __grid_constant__ fields_dev F_,
                                                          const __grid_constant__ CUtensorMap tmu,
                                                          const __grid_constant__ CUtensorMap tmv,
                                                          const __grid_constant__ CUtensorMap tmw, const double *lx,
                                                          const double *ly, const double *lz, double cdt,
                                                          const double *time_p, int var_den, int tz, int *err) {
+    const fields_dev *__restrict__ F = &F_;
     extern __shared__ __align__(128) unsigned char ev_smem[];
     double *ring = reinterpret_cast<double *>(ev_smem);  // [kEvRing][3][kEvH][kEvW]
     uint64_t *bar = reinterpret_cast<uint64_t *>(ev_smem + (size_t)kEvRing * 3 * kEvPlaneBytes);
@@ -811,7 +816,7 @@ bool edge_vel_tensor_map(const grid_dev &g, const double *base, CUtensorMap *out
 }
 
 // launch of k_edge_vel_tma over the interior: z chunks of tz planes
-void launch_edge_vel_tma(const grid_dev &g, const fields_dev *F, const CUtensorMap tm[3], const double *lx,
+void launch_edge_vel_tma(const grid_dev &g, const fields_dev &F, const CUtensorMap tm[3], const double *lx,
                          const double *ly, const double *lz, double cdt, const double *time_p, int var_den, int *err,
                          cudaStream_t st) {
     static bool attr = false;
@@ -866,7 +871,8 @@ __device__ inline void set_refmap(double norml, double normr, double &ml, double
 }
 
 template <typename FT>
-__global__ void k_upwind(grid_dev g, const fields_dev *__restrict__ F) {
+__global__ void k_upwind(grid_dev g, const __grid_constant__ fields_dev F_) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -929,14 +935,15 @@ __global__ void k_upwind(grid_dev g, const fields_dev *__restrict__ F) {
         fr[2][nb] = wr;
     }
 }
-template __global__ void k_upwind<double>(grid_dev, const fields_dev *__restrict__);
-template __global__ void k_upwind<float>(grid_dev, const fields_dev *__restrict__);
+template __global__ void k_upwind<double>(grid_dev, const __grid_constant__ fields_dev);
+template __global__ void k_upwind<float>(grid_dev, const __grid_constant__ fields_dev);
 
 // -------------------------------------------------------------------------
 // MAC projection: rhs (fill_mac_rhs, fluid_3d.cc:2244-2265), solution
 // extraction (:2268-2281) and face correction (subtract_q_grad, :2284-2304).
 // -------------------------------------------------------------------------
-__global__ void k_mac_rhs(grid_dev g, const fields_dev *__restrict__ F, double *r, double cdt) {
+__global__ void k_mac_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, double cdt) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int j = blockIdx.y * blockDim.y + threadIdx.y;
     int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -948,7 +955,8 @@ __global__ void k_mac_rhs(grid_dev g, const fields_dev *__restrict__ F, double *
     r[i + g.sm * (j + g.sn * k)] = s;
 }
 
-__global__ void k_mac_extract(grid_dev g, const fields_dev *__restrict__ F, const double *x) {
+__global__ void k_mac_extract(grid_dev g, const __grid_constant__ fields_dev F_, const double *x) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int j = blockIdx.y * blockDim.y + threadIdx.y;
     int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -956,7 +964,8 @@ __global__ void k_mac_extract(grid_dev g, const fields_dev *__restrict__ F, cons
     F->q[gidx(g, i + 2, j + 2, k + 2)] = x[i + g.sm * (j + g.sn * k)];
 }
 
-__global__ void k_sub_qgrad(grid_dev g, const fields_dev *__restrict__ F, double cdt, int var_den) {
+__global__ void k_sub_qgrad(grid_dev g, const __grid_constant__ fields_dev F_, double cdt, int var_den) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
     int k = blockIdx.z * blockDim.z + threadIdx.z + 2;
@@ -985,9 +994,10 @@ __global__ void k_sub_qgrad(grid_dev g, const fields_dev *__restrict__ F, double
 // Explicit momentum update, fluid_3d::compute_ustar (fluid_3d.cc:1309-1352).
 // -------------------------------------------------------------------------
 template <typename FT>
-__global__ void __launch_bounds__(256, 3) k_ustar(grid_dev g, const fields_dev *__restrict__ F, const double *lx,
+__global__ void __launch_bounds__(256, 3) k_ustar(grid_dev g, const __grid_constant__ fields_dev F_, const double *lx,
                                                   const double *ly, const double *lz, double cdt,
                                                   const double *time_p, int var_den) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
     int k = blockIdx.z * blockDim.z + threadIdx.z + 2;
@@ -1029,9 +1039,9 @@ __global__ void __launch_bounds__(256, 3) k_ustar(grid_dev g, const fields_dev *
         F->vel[d][ind] += dd;
     }
 }
-template __global__ void k_ustar<double>(grid_dev, const fields_dev *__restrict__, const double *, const double *,
+template __global__ void k_ustar<double>(grid_dev, const __grid_constant__ fields_dev, const double *, const double *,
                                          const double *, double, const double *, int);
-template __global__ void k_ustar<float>(grid_dev, const fields_dev *__restrict__, const double *, const double *,
+template __global__ void k_ustar<float>(grid_dev, const __grid_constant__ fields_dev, const double *, const double *,
                                         const double *, double, const double *, int);
 
 // -------------------------------------------------------------------------
@@ -1045,7 +1055,8 @@ __device__ inline bool elem_in_domain(const grid_dev &g, int ei, int ej, int ek)
            (g.prd[2] || (ek >= 0 && ek <= g.so - 1));
 }
 
-__global__ void k_fem_rhs(grid_dev g, const fields_dev *__restrict__ F, double *r, gradphi_t gp) {
+__global__ void k_fem_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, gradphi_t gp) {
+    const fields_dev *__restrict__ F = &F_;
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     int b = blockIdx.y * blockDim.y + threadIdx.y;
     int c = blockIdx.z * blockDim.z + threadIdx.z;
@@ -1107,7 +1118,8 @@ __global__ void k_fem_rhs(grid_dev g, const fields_dev *__restrict__ F, double *
 }
 
 // p += x - mean, dp = x - mean over FEM nodes (extract_pp_soln, :2685-2712)
-__global__ void k_fem_extract(grid_dev g, const fields_dev *__restrict__ F, const double *x, const double *mean) {
+__global__ void k_fem_extract(grid_dev g, const __grid_constant__ fields_dev F_, const double *x, const double *mean) {
+    const fields_dev *__restrict__ F = &F_;
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     int b = blockIdx.y * blockDim.y + threadIdx.y;
     int c = blockIdx.z * blockDim.z + threadIdx.z;
@@ -1120,7 +1132,8 @@ __global__ void k_fem_extract(grid_dev g, const fields_dev *__restrict__ F, cons
 }
 
 // u, dvel -= dt grad(dp), subtract_pres_grad (:2717-2753) with neg_pres_dgrad
-__global__ void k_sub_pgrad(grid_dev g, const fields_dev *__restrict__ F, double dt, int var_den) {
+__global__ void k_sub_pgrad(grid_dev g, const __grid_constant__ fields_dev F_, double dt, int var_den) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
     int k = blockIdx.z * blockDim.z + threadIdx.z + 2;

@@ -16,7 +16,8 @@ __device__ inline double mphi(const grid_dev &g, const objmap_dev &m, int o, int
 // (fields.hh:572-592, non-TANG): for the primary map of every interior cell
 // and for extrapolated maps that abut a primary map orthogonally.
 // -------------------------------------------------------------------------
-__global__ void __launch_bounds__(256, 3) k_edge_refmap(grid_dev g, const fields_dev *__restrict__ F, double cdt, int *err) {
+__global__ void __launch_bounds__(256, 3) k_edge_refmap(grid_dev g, const __grid_constant__ fields_dev F_, double cdt, int *err) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
     int k = blockIdx.z * blockDim.z + threadIdx.z + 2;
@@ -31,19 +32,19 @@ __global__ void __launch_bounds__(256, 3) k_edge_refmap(grid_dev g, const fields
     for (int c = 0; c < 3; c++) vel[c] = F->vel[c][ind];
     for (int o = 0; o < g.n_obj; o++) {
         const objmap_dev &m = F->om[o];
-        int cd = m.code[ind];
+        int cd = F->code[o][ind];
         if (cd < 0) continue;
         if (cd > 0) {  // ref_map::abut_primary (fields.hh:466-477)
             bool ab = false;
             for (int d = 0; d < 3 && !ab; d++)
-                if (m.code[ind + strides[d]] == 0 || m.code[ind - strides[d]] == 0) ab = true;
+                if (F->code[o][ind + strides[d]] == 0 || F->code[o][ind - strides[d]] == 0) ab = true;
             if (!ab) continue;
         }
         double nv[3][3];
         for (int d = 0; d < 3; d++) {
             int s = strides[d];
             int q[5] = {ind - 2 * s, ind - s, ind, ind + s, ind + 2 * s};
-            if (m.code[q[0]] < 0 || m.code[q[1]] < 0 || m.code[q[3]] < 0 || m.code[q[4]] < 0) {
+            if (F->code[o][q[0]] < 0 || F->code[o][q[1]] < 0 || F->code[o][q[3]] < 0 || F->code[o][q[4]] < 0) {
                 atomicAdd(err, 1);  // missing cells for the finite differences (:668-676)
                 return;
             }
@@ -69,7 +70,8 @@ __global__ void __launch_bounds__(256, 3) k_edge_refmap(grid_dev g, const fields
 // advective increment from the MAC-projected face velocities and the
 // upwinded face maps.  Interior cells with a primary map.
 // -------------------------------------------------------------------------
-__global__ void k_refmap_predict(grid_dev g, const fields_dev *__restrict__ F, double cdt) {
+__global__ void k_refmap_predict(grid_dev g, const __grid_constant__ fields_dev F_, double cdt) {
+    const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
     int k = blockIdx.z * blockDim.z + threadIdx.z + 2;
@@ -77,7 +79,7 @@ __global__ void k_refmap_predict(grid_dev g, const fields_dev *__restrict__ F, d
     const int ind = gidx(g, i, j, k);
     for (int o = 0; o < g.n_obj; o++) {
         const objmap_dev &m = F->om[o];
-        if (m.code[ind] != 0) continue;
+        if (F->code[o][ind] != 0) continue;
         double avgs[3];
         avgs[0] = -0.5 * cdt * (face_ld(g, F, 0, ind) + face_ld(g, F, 3, ind)) * g.dxsp;
         avgs[1] = -0.5 * cdt * (face_ld(g, F, 7, ind) + face_ld(g, F, 10, ind)) * g.dysp;
@@ -95,17 +97,18 @@ __global__ void k_refmap_predict(grid_dev g, const fields_dev *__restrict__ F, d
 // extrapolation starts), the pass also sets the extrapolation's layer tags
 // and claims as k_lay_init would from the reset codes: primary cells 0,
 // every other cell free.
-__global__ void k_snapshot_reset(grid_dev g, const fields_dev *__restrict__ F, uint8_t *lay, int *inl) {
+__global__ void k_snapshot_reset(grid_dev g, const __grid_constant__ fields_dev F_, uint8_t *lay, int *inl) {
+    const fields_dev *__restrict__ F = &F_;
     int ind = blockIdx.x * blockDim.x + threadIdx.x;
     if (ind >= g.ncell) return;
     for (int o = 0; o < g.n_obj; o++) {
         const objmap_dev &m = F->om[o];
-        int cd = m.code[ind];
+        int cd = F->code[o][ind];
         m.code_prev[ind] = (cd > 0) ? cd : -1;
         if (cd > 0) {
             for (int c = 0; c < 3; c++) m.x_prev[c][ind] = m.x[c][ind];
             for (int c = 0; c < 9; c++) m.gp_prev[c][ind] = m.gp[c][ind];
-            m.code[ind] = -1;
+            F->code[o][ind] = -1;
         }
         if (lay) {
             lay[(size_t)o * g.ncell + ind] = (cd == 0) ? 0 : 255;
@@ -115,7 +118,8 @@ __global__ void k_snapshot_reset(grid_dev g, const fields_dev *__restrict__ F, u
 }
 
 // extraps.reset() alone (init_iter, fluid_3d.cc:270)
-__global__ void k_reset_extraps(grid_dev g, const fields_dev *__restrict__ F) {
+__global__ void k_reset_extraps(grid_dev g, const __grid_constant__ fields_dev F_) {
+    const fields_dev *__restrict__ F = &F_;
     int ind = blockIdx.x * blockDim.x + threadIdx.x;
     if (ind >= g.ncell) return;
     for (int o = 0; o < g.n_obj; o++)
@@ -151,7 +155,8 @@ __device__ inline bool inner_ghost(const grid_dev &g, int i, int j, int k) {
 // writes only its own maps), so all of them advance one layer per launch.
 
 // first_layer + mark_primary (fluid_3d_ex.cc:52-70): reset the layer tags
-__global__ void k_lay_init(grid_dev g, const fields_dev *__restrict__ F, uint8_t *lay, int *inl) {
+__global__ void k_lay_init(grid_dev g, const __grid_constant__ fields_dev F_, uint8_t *lay, int *inl) {
+    const fields_dev *__restrict__ F = &F_;
     int ind = blockIdx.x * blockDim.x + threadIdx.x;
     if (ind >= g.ncell) return;
     for (int o = 0; o < g.n_obj; o++) {
@@ -528,14 +533,17 @@ __device__ inline bool ls_first(const int (&cd)[4], const double (&xv)[4][3], in
 // Every object's frontier in one launch: lane group w (LANES lanes)
 // takes entry w of the concatenated frontiers.  The weights wt^n (n = |p|+|q|+|r|) come from a
 // per-block table of the same pow() values.
-// The first npush blocks list the next layer's cells instead (push_layer;
-// next 0: none): they read the same lists and write what no fit reads.
+// The first npush blocks list the next layer's cells instead (push_layer):
+// they read the same lists and write what no fit reads; zcnt, the lengths of
+// the lists after those, is zeroed for the next launch.
 template <int LANES>
-__global__ void __launch_bounds__(128) k_extrap_layer(grid_dev g, const fields_dev *__restrict__ F, const int *front,
+__global__ void __launch_bounds__(128) k_extrap_layer(grid_dev g, const __grid_constant__ fields_dev F_, const int *front,
                                                       const int *cnt, int L, int max_rs, double wt, const double *lx,
                                                       const double *ly, const double *lz, int *err, int npush,
-                                                      uint8_t *lay, int *inl, int next, int *nfront, int *ncnt) {
+                                                      uint8_t *lay, int *inl, int next, int *nfront, int *ncnt, int *zcnt) {
+    const fields_dev *__restrict__ F = &F_;
     if ((int)blockIdx.x < npush) {
+        if (blockIdx.x == 0 && threadIdx.x < kMaxObj) zcnt[threadIdx.x] = 0;
         push_layer(g, front, cnt, lay, inl, next, nfront, ncnt, blockIdx.x * blockDim.x + threadIdx.x,
                    npush * blockDim.x);
         return;
@@ -650,17 +658,18 @@ __global__ void __launch_bounds__(128) k_extrap_layer(grid_dev g, const fields_d
     }
 }
 
-template __global__ void k_extrap_layer<4>(grid_dev, const fields_dev *__restrict__, const int *, const int *, int,
+template __global__ void k_extrap_layer<4>(grid_dev, const __grid_constant__ fields_dev, const int *, const int *, int,
                                             int, double, const double *, const double *, const double *, int *, int,
-                                            uint8_t *, int *, int, int *, int *);
-template __global__ void k_extrap_layer<32>(grid_dev, const fields_dev *__restrict__, const int *, const int *, int,
+                                            uint8_t *, int *, int, int *, int *, int *);
+template __global__ void k_extrap_layer<32>(grid_dev, const __grid_constant__ fields_dev, const int *, const int *, int,
                                              int, double, const double *, const double *, const double *, int *, int,
-                                             uint8_t *, int *, int, int *, int *);
+                                             uint8_t *, int *, int, int *, int *, int *);
 
 // communicate_a_layer on one rank (fluid_3d_comm.cc:203-280): image-backed
 // ghosts receive the maps of the layer just made at their image (periodic
 // domains only).
-__global__ void k_layer_ghost_copy(grid_dev g, const fields_dev *__restrict__ F, int L) {
+__global__ void k_layer_ghost_copy(grid_dev g, const __grid_constant__ fields_dev F_, int L) {
+    const fields_dev *__restrict__ F = &F_;
     int ind = blockIdx.x * blockDim.x + threadIdx.x;
     if (ind >= g.ncell) return;
     int k = ind / g.smn4, j = (ind % g.smn4) / g.sm4, i = ind % g.sm4;
@@ -688,12 +697,13 @@ __global__ void k_layer_ghost_copy(grid_dev g, const fields_dev *__restrict__ F,
 // primary x = (x + xpred)/2; extrapolated maps average with the previous
 // extrapolation of the same object, or take xpred where none existed.
 // -------------------------------------------------------------------------
-__global__ void k_refmap_correct(grid_dev g, const fields_dev *__restrict__ F, int *prob, int var_den) {
+__global__ void k_refmap_correct(grid_dev g, const __grid_constant__ fields_dev F_, int *prob, int var_den) {
+    const fields_dev *__restrict__ F = &F_;
     int ind = blockIdx.x * blockDim.x + threadIdx.x;
     if (ind >= g.ncell) return;
     for (int o = 0; o < g.n_obj; o++) {
         const objmap_dev &m = F->om[o];
-        int cd = m.code[ind];
+        int cd = F->code[o][ind];
         if (cd < 0) continue;
         if (cd == 0) {
             for (int c = 0; c < 3; c++) m.x[c][ind] = 0.5 * (m.x[c][ind] + m.xp[c][ind]);
@@ -711,12 +721,13 @@ __global__ void k_refmap_correct(grid_dev g, const fields_dev *__restrict__ F, i
 }
 
 // revert_reference_map_update (fluid_3d.cc:1257-1283)
-__global__ void k_refmap_revert(grid_dev g, const fields_dev *__restrict__ F) {
+__global__ void k_refmap_revert(grid_dev g, const __grid_constant__ fields_dev F_) {
+    const fields_dev *__restrict__ F = &F_;
     int ind = blockIdx.x * blockDim.x + threadIdx.x;
     if (ind >= g.ncell) return;
     for (int o = 0; o < g.n_obj; o++) {
         const objmap_dev &m = F->om[o];
-        int cd = m.code[ind];
+        int cd = F->code[o][ind];
         if (cd == 0) {
             for (int c = 0; c < 3; c++) m.x[c][ind] = 2 * m.x[c][ind] - m.xp[c][ind];
         } else if (cd > 0 && m.code_prev[ind] > 0) {
@@ -727,12 +738,13 @@ __global__ void k_refmap_revert(grid_dev g, const fields_dev *__restrict__ F) {
 
 // update_reference_map_full (fluid_3d.cc:1285-1306): x = xpred everywhere,
 // then its update_rho (:1304) from this cell's maps
-__global__ void k_refmap_full(grid_dev g, const fields_dev *__restrict__ F, int var_den) {
+__global__ void k_refmap_full(grid_dev g, const __grid_constant__ fields_dev F_, int var_den) {
+    const fields_dev *__restrict__ F = &F_;
     int ind = blockIdx.x * blockDim.x + threadIdx.x;
     if (ind >= g.ncell) return;
     for (int o = 0; o < g.n_obj; o++) {
         const objmap_dev &m = F->om[o];
-        if (m.code[ind] < 0) continue;
+        if (F->code[o][ind] < 0) continue;
         for (int c = 0; c < 3; c++) m.x[c][ind] = m.xp[c][ind];
     }
     if (var_den) F->rho[ind] = cell_rho(g, F, ind);
@@ -740,7 +752,8 @@ __global__ void k_refmap_full(grid_dev g, const fields_dev *__restrict__ F, int 
 
 // x = xpred for the maps of one extrapolation (init_extrapolate,
 // fluid_3d_ex.cc:16-27)
-__global__ void k_extraps_full(grid_dev g, const fields_dev *__restrict__ F) {
+__global__ void k_extraps_full(grid_dev g, const __grid_constant__ fields_dev F_) {
+    const fields_dev *__restrict__ F = &F_;
     int ind = blockIdx.x * blockDim.x + threadIdx.x;
     if (ind >= g.ncell) return;
     for (int o = 0; o < g.n_obj; o++) {
@@ -756,13 +769,14 @@ __global__ void k_extraps_full(grid_dev g, const fields_dev *__restrict__ F) {
 // map of layer nlayers+1); a first-layer extrapolated map with negative level
 // set enters it.
 // -------------------------------------------------------------------------
-__global__ void k_redraw(grid_dev g, const fields_dev *__restrict__ F, int nlayers, int *fatal) {
+__global__ void k_redraw(grid_dev g, const __grid_constant__ fields_dev F_, int nlayers, int *fatal) {
+    const fields_dev *__restrict__ F = &F_;
     int ind = blockIdx.x * blockDim.x + threadIdx.x;
     if (ind >= g.ncell) return;
     bool occupied = false;
     int prim = -1;
     for (int o = 0; o < g.n_obj; o++)
-        if (F->om[o].code[ind] == 0) prim = o;
+        if (F->code[o][ind] == 0) prim = o;
     int moved_out = -1;
     if (prim >= 0) {
         const objmap_dev &m = F->om[prim];
@@ -780,7 +794,7 @@ __global__ void k_redraw(grid_dev g, const fields_dev *__restrict__ F, int nlaye
         for (int o = 0; o < g.n_obj; o++) {
             if ((pass == 0) == (o == moved_out)) continue;
             const objmap_dev &m = F->om[o];
-            int cd = m.code[ind];
+            int cd = F->code[o][ind];
             if (cd <= 0) continue;
             double sp = mphi(g, m, o, ind);
             bool inside = (sp < 0 && cd == 1);
@@ -788,7 +802,7 @@ __global__ void k_redraw(grid_dev g, const fields_dev *__restrict__ F, int nlaye
             double pp = (prim >= 0) ? mphi(g, F->om[prim], prim, ind) : nan("");
             if ((occupied && sp < pp) || !occupied) {
                 if (pp < -g.dx) atomicAdd(fatal, 1);
-                if (prim >= 0) F->om[prim].code[ind] = -1;  // overwritten primary map
+                if (prim >= 0) F->code[prim][ind] = -1;  // overwritten primary map
                 m.code[ind] = 0;
                 prim = o;
                 occupied = true;

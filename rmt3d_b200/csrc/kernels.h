@@ -45,29 +45,29 @@ struct gradphi_t {
 
 __global__ void k_periodic_copy(grid_dev g, ptr_list pl, int corner);
 __global__ void k_bc_cc(grid_dev g, int n, bc_face lo, bc_face hi, double *u, double *v, double *w);
-__global__ void k_bc_cf(grid_dev g, int walls, bc_faces bcs, const fields_dev *F);
-__global__ void k_stress(grid_dev g, const fields_dev *__restrict__ F, const int *list, const int *cnt);
-__global__ void k_stress_fluid(grid_dev g, const fields_dev *__restrict__ F, int *list, int *cnt);
+__global__ void k_bc_cf(grid_dev g, int walls, bc_faces bcs, const __grid_constant__ fields_dev F_);
+__global__ void k_stress(grid_dev g, const __grid_constant__ fields_dev F_, const int *list, const int *cnt);
+__global__ void k_stress_fluid(grid_dev g, const __grid_constant__ fields_dev F_, int *list, int *cnt);
 // FT: the face states' type: float in the FP32-advection form (RMT3D_MIXED_BULK32), else double
 template <typename FT>
-__global__ void k_edge_vel(grid_dev g, const fields_dev *__restrict__ F, const double *lx, const double *ly,
+__global__ void k_edge_vel(grid_dev g, const __grid_constant__ fields_dev F_, const double *lx, const double *ly,
                            const double *lz, double cdt, const double *time_p, int var_den);
 // the velocity edge states with TMA-staged velocity tiles (k_fluid.cu)
 bool edge_vel_tensor_map(const grid_dev &g, const double *base, CUtensorMap *out);
-void launch_edge_vel_tma(const grid_dev &g, const fields_dev *F, const CUtensorMap tm[3], const double *lx,
+void launch_edge_vel_tma(const grid_dev &g, const fields_dev &F, const CUtensorMap tm[3], const double *lx,
                          const double *ly, const double *lz, double cdt, const double *time_p, int var_den, int *err,
                          cudaStream_t st);
 template <typename FT>
-__global__ void k_upwind(grid_dev g, const fields_dev *__restrict__ F);
-__global__ void k_mac_rhs(grid_dev g, const fields_dev *__restrict__ F, double *r, double cdt);
-__global__ void k_mac_extract(grid_dev g, const fields_dev *__restrict__ F, const double *x);
-__global__ void k_sub_qgrad(grid_dev g, const fields_dev *__restrict__ F, double cdt, int var_den);
+__global__ void k_upwind(grid_dev g, const __grid_constant__ fields_dev F_);
+__global__ void k_mac_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, double cdt);
+__global__ void k_mac_extract(grid_dev g, const __grid_constant__ fields_dev F_, const double *x);
+__global__ void k_sub_qgrad(grid_dev g, const __grid_constant__ fields_dev F_, double cdt, int var_den);
 template <typename FT>
-__global__ void k_ustar(grid_dev g, const fields_dev *__restrict__ F, const double *lx, const double *ly,
+__global__ void k_ustar(grid_dev g, const __grid_constant__ fields_dev F_, const double *lx, const double *ly,
                         const double *lz, double cdt, const double *time_p, int var_den);
-__global__ void k_fem_rhs(grid_dev g, const fields_dev *__restrict__ F, double *r, gradphi_t gp);
-__global__ void k_fem_extract(grid_dev g, const fields_dev *__restrict__ F, const double *x, const double *mean);
-__global__ void k_sub_pgrad(grid_dev g, const fields_dev *__restrict__ F, double dt, int var_den);
+__global__ void k_fem_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, gradphi_t gp);
+__global__ void k_fem_extract(grid_dev g, const __grid_constant__ fields_dev F_, const double *x, const double *mean);
+__global__ void k_sub_pgrad(grid_dev g, const __grid_constant__ fields_dev F_, double dt, int var_den);
 __global__ void k_chk_pack(grid_dev g, const fields_dev *__restrict__ F, double *__restrict__ buf);
 __global__ void k_macro_cells(grid_dev g, const fields_dev *__restrict__ F, const double *lz, int var_den,
                               double *out, unsigned *ticket);

@@ -117,7 +117,9 @@ struct rmt3d_scene {
     rmt3d_scene_desc d;
     grid_dev g;
     fields_dev hF;
-    fields_dev *dF = nullptr;
+    objmap_dev hom[kMaxObj] = {};  // the objects' maps: host copy of the table hF.om
+    objmap_dev *dom = nullptr;
+    fields_dev *dF = nullptr;      // hF in device memory, for the kernels off the step
     cudaStream_t st = 0;
     bool own_stream = false;
     std::vector<void *> allocs;
@@ -141,7 +143,7 @@ struct rmt3d_scene {
     uint8_t *lay = nullptr;  // per object: layer tags
     int *inl = nullptr;      // per object: layer that claimed the cell (0: none)
     int *front[2] = {nullptr, nullptr};  // per object: ncell entries each
-    int *fcnt = nullptr;                  // frontier lengths, [nlayers][kMaxObj]
+    int *fcnt = nullptr;                  // frontier lengths, [3][kMaxObj]
     // lanes per frontier cell of the least-squares extrapolation: a warp when
     // the scene steps on its own, 4 when it steps inside a group with others
     int extrap_lanes = 32;
@@ -339,7 +341,7 @@ static void fill_boundary_cf(rmt3d_scene *s) {
     if (walls) {
         const int mx = std::max(g.sm4, std::max(g.sn4, g.so4));
         dim3 gr((mx + 31) / 32, (mx + 7) / 8, 6);
-        k_bc_cf<<<gr, dim3(32, 8, 1), 0, s->st>>>(g, walls, bcs, s->dF);
+        k_bc_cf<<<gr, dim3(32, 8, 1), 0, s->st>>>(g, walls, bcs, s->hF);
         s->count();
     }
     if (g.prd[0] || g.prd[1] || g.prd[2]) {
@@ -370,7 +372,7 @@ static void comm_face_maps(rmt3d_scene *s) {
         pl.n = 18;
         pl.ni = 0;
         pl.nf = 0;
-        for (int a = 0; a < 18; a++) pl.p[a] = s->hF.om[o].fx[a];
+        for (int a = 0; a < 18; a++) pl.p[a] = s->hom[o].fx[a];
         k_periodic_copy<<<grd(g.sm4, g.sn4, g.so4), blk(), 0, s->st>>>(g, pl, 0);
         s->count();
     }
@@ -381,7 +383,7 @@ static void comm_primary(rmt3d_scene *s) {
     const grid_dev &g = s->g;
     if (!(g.prd[0] || g.prd[1] || g.prd[2])) return;
     for (int o = 0; o < g.n_obj; o++) {
-        objmap_dev &m = s->hF.om[o];
+        objmap_dev &m = s->hom[o];
         ptr_list pl;
         pl.n = 0;
         pl.nf = 0;
@@ -407,13 +409,14 @@ static void extrapolate(rmt3d_scene *s, bool lay_ready = false) {
     // without a periodic axis no ghost cell is the image of an interior
     // cell, and the two ghost-copy kernels would find nothing to do
     const bool prd = g.prd[0] || g.prd[1] || g.prd[2];
-    // a list length per layer, all zeroed at once
-    auto cnt = [&](int layer) { return s->fcnt + (layer - 1) * kMaxObj; };
+    // the list lengths of the layer being fitted, of the one being listed, and
+    // of the one after, which the launch zeroes
+    auto cnt = [&](int layer) { return s->fcnt + (layer % 3) * kMaxObj; };
     if (!lay_ready) {
-        k_lay_init<<<nb, 256, 0, s->st>>>(g, s->dF, s->lay, s->inl);
+        k_lay_init<<<nb, 256, 0, s->st>>>(g, s->hF, s->lay, s->inl);
         s->count();
     }
-    cudaMemsetAsync(s->fcnt, 0, s->d.nlayers * kMaxObj * sizeof(int), s->st);
+    cudaMemsetAsync(s->fcnt, 0, 3 * kMaxObj * sizeof(int), s->st);
     k_lay_push<<<nb, 256, 0, s->st>>>(g, s->lay, s->inl, s->front[0], cnt(1));
     s->count();
     if (prd) {
@@ -426,13 +429,13 @@ static void extrapolate(rmt3d_scene *s, bool lay_ready = false) {
         const bool more = L < s->d.nlayers;
         const int npush = more ? 148 : 0;
         auto kern = s->extrap_lanes == 4 ? k_extrap_layer<4> : k_extrap_layer<32>;
-        kern<<<npush + per_warp_blocks, 128, 0, s->st>>>(g, s->dF, s->front[cur], cnt(L), L, s->d.max_extrap_rs,
+        kern<<<npush + per_warp_blocks, 128, 0, s->st>>>(g, s->hF, s->front[cur], cnt(L), L, s->d.max_extrap_rs,
                                                          s->d.weight_fac, s->lx, s->ly, s->lz, s->counters + 2, npush,
                                                          s->lay, s->inl, L + 1, s->front[cur ^ 1],
-                                                         more ? cnt(L + 1) : nullptr);
+                                                         cnt(L + 1), cnt(L + 2));
         s->count();
         if (prd) {
-            k_layer_ghost_copy<<<nb, 256, 0, s->st>>>(g, s->dF, L);
+            k_layer_ghost_copy<<<nb, 256, 0, s->st>>>(g, s->hF, L);
             s->count();
         }
         if (more && prd) {
@@ -794,7 +797,7 @@ static void update_rinv(rmt3d_scene *s) {
 static void init_extrapolate(rmt3d_scene *s) {
     if (s->g.n_obj == 0) return;
     extrapolate(s);
-    k_extraps_full<<<lin_blocks(s->g.ncell), 256, 0, s->st>>>(s->g, s->dF);
+    k_extraps_full<<<lin_blocks(s->g.ncell), 256, 0, s->st>>>(s->g, s->hF);
     s->count();
 }
 
@@ -815,11 +818,11 @@ static void compute_stress(rmt3d_scene *s) {
     const grid_dev &g = s->g;
     const bool maps = g.n_obj > 0;
     if (maps) cudaMemsetAsync(s->mcnt, 0, sizeof(int), s->st);
-    k_stress_fluid<<<grd_of(s->bshape, g.sm + 4, g.sn + 4, g.so + 4), blk_of(s->bshape), 0, s->st>>>(g, s->dF, maps ? s->mlist : nullptr,
+    k_stress_fluid<<<grd_of(s->bshape, g.sm + 4, g.sn + 4, g.so + 4), blk_of(s->bshape), 0, s->st>>>(g, s->hF, maps ? s->mlist : nullptr,
                                                                           s->mcnt);
     s->count();
     if (maps) {
-        k_stress<<<148 * 8, 128, 0, s->st>>>(g, s->dF, s->mlist, s->mcnt);
+        k_stress<<<148 * 8, 128, 0, s->st>>>(g, s->hF, s->mlist, s->mcnt);
         s->count();
     }
 }
@@ -848,17 +851,17 @@ static void advance_half(rmt3d_scene *s) {
 static void ph_edges(rmt3d_scene *s) {
     const grid_dev &g = s->g;
     if (s->edge_tma)
-        launch_edge_vel_tma(g, s->dF, s->tm_vel, s->lx, s->ly, s->lz, s->dt, &s->ctl->time, s->d.var_den,
+        launch_edge_vel_tma(g, s->hF, s->tm_vel, s->lx, s->ly, s->lz, s->dt, &s->ctl->time, s->d.var_den,
                             s->counters + 7, s->st);
     else if (g.f32face)
-        k_edge_vel<float><<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->dF, s->lx, s->ly, s->lz, s->dt,
+        k_edge_vel<float><<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->lx, s->ly, s->lz, s->dt,
                                                                        &s->ctl->time, s->d.var_den);
     else
-        k_edge_vel<double><<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->dF, s->lx, s->ly, s->lz, s->dt,
+        k_edge_vel<double><<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->lx, s->ly, s->lz, s->dt,
                                                                         &s->ctl->time, s->d.var_den);
     s->count();
     if (g.n_obj > 0) {
-        k_edge_refmap<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->dF, s->dt, s->counters + 5);
+        k_edge_refmap<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->dt, s->counters + 5);
         s->count();
     }
     advance_half(s);
@@ -869,8 +872,8 @@ static void ph_upwind(rmt3d_scene *s) {
     const grid_dev &g = s->g;
     fill_boundary_cf(s);
     comm_face_maps(s);
-    if (g.f32face) k_upwind<float><<<grd_of(s->bshape, g.sm + 1, g.sn + 1, g.so + 1), blk_of(s->bshape), 0, s->st>>>(g, s->dF);
-    else k_upwind<double><<<grd_of(s->bshape, g.sm + 1, g.sn + 1, g.so + 1), blk_of(s->bshape), 0, s->st>>>(g, s->dF);
+    if (g.f32face) k_upwind<float><<<grd_of(s->bshape, g.sm + 1, g.sn + 1, g.so + 1), blk_of(s->bshape), 0, s->st>>>(g, s->hF);
+    else k_upwind<double><<<grd_of(s->bshape, g.sm + 1, g.sn + 1, g.so + 1), blk_of(s->bshape), 0, s->st>>>(g, s->hF);
     s->count();
     fill_boundary_cf(s);
 }
@@ -882,16 +885,16 @@ static void ph_upwind(rmt3d_scene *s) {
 static void ph_mac_pre(rmt3d_scene *s, double cdt) {
     const grid_dev &g = s->g;
     update_rinv(s);
-    k_mac_rhs<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->dF, s->mac.rhs(), cdt);
+    k_mac_rhs<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->mac.rhs(), cdt);
     s->count();
 }
 
 static void ph_mac_post(rmt3d_scene *s, double cdt) {
     const grid_dev &g = s->g;
-    k_mac_extract<<<grd(g.sm, g.sn, g.so), blk(), 0, s->st>>>(g, s->dF, s->mac.sol());
+    k_mac_extract<<<grd(g.sm, g.sn, g.so), blk(), 0, s->st>>>(g, s->hF, s->mac.sol());
     s->count();
     comm_pressure(s);
-    k_sub_qgrad<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->dF, cdt, s->d.var_den);
+    k_sub_qgrad<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, cdt, s->d.var_den);
     s->count();
     fill_boundary_cf(s);
 }
@@ -903,18 +906,18 @@ static void ph_refmap(rmt3d_scene *s, double cdt) {
     // without a periodic axis nothing changes the codes between the snapshot
     // and the extrapolation, so the snapshot pass sets the layer tags too
     const bool prd = g.prd[0] || g.prd[1] || g.prd[2];
-    k_refmap_predict<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->dF, cdt);
-    k_snapshot_reset<<<lin_blocks(g.ncell), 256, 0, s->st>>>(g, s->dF, prd ? nullptr : s->lay, s->inl);
+    k_refmap_predict<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, cdt);
+    k_snapshot_reset<<<lin_blocks(g.ncell), 256, 0, s->st>>>(g, s->hF, prd ? nullptr : s->lay, s->inl);
     s->count(2);
     comm_primary(s);
     extrapolate(s, !prd);
     // update_rho follows in the same pass (var_den)
-    k_refmap_correct<<<lin_blocks(g.ncell), 256, 0, s->st>>>(g, s->dF, s->counters + 3, s->d.var_den);
+    k_refmap_correct<<<lin_blocks(g.ncell), 256, 0, s->st>>>(g, s->hF, s->counters + 3, s->d.var_den);
     s->count();
 }
 
 static void ph_revert(rmt3d_scene *s) {
-    k_refmap_revert<<<lin_blocks(s->g.ncell), 256, 0, s->st>>>(s->g, s->dF);
+    k_refmap_revert<<<lin_blocks(s->g.ncell), 256, 0, s->st>>>(s->g, s->hF);
     s->count();
 }
 
@@ -922,10 +925,10 @@ static void ph_revert(rmt3d_scene *s) {
 static void ph_ustar(rmt3d_scene *s) {
     const grid_dev &g = s->g;
     if (g.f32face)
-        k_ustar<float><<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->dF, s->lx, s->ly, s->lz, s->dt,
+        k_ustar<float><<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->lx, s->ly, s->lz, s->dt,
                                                                     &s->ctl->time, s->d.var_den);
     else
-        k_ustar<double><<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->dF, s->lx, s->ly, s->lz, s->dt,
+        k_ustar<double><<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->lx, s->ly, s->lz, s->dt,
                                                                      &s->ctl->time, s->d.var_den);
     s->count();
     fill_boundary_cc(s);
@@ -969,10 +972,15 @@ __global__ void k_mean(const double *x, size_t n, double scale, double *out, uns
         }
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        const volatile double *part = out + 1;
+    if (!last) return;
+    // the whole block fetches the partials, one thread adds them in block order
+    __shared__ double part[kMeanBlocks];
+    __threadfence();
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) part[b] = __ldcg(out + 1 + b);
+    __syncthreads();
+    if (threadIdx.x == 0) {
         double t = 0;
+#pragma unroll 4
         for (unsigned b = 0; b < gridDim.x; b++) t += part[b];
         out[0] = t;
         *ticket = 0;
@@ -985,7 +993,7 @@ static void ph_pp_pre(rmt3d_scene *s) {
     // the density is already that of the current maps: update_rho ran after
     // the reference-map update, and nothing since has moved a map
     update_rinv(s);
-    k_fem_rhs<<<grd_of(s->bshape, g.fm, g.fn, g.fo), blk_of(s->bshape), 0, s->st>>>(g, s->dF, s->fem.rhs(), s->gradphi);
+    k_fem_rhs<<<grd_of(s->bshape, g.fm, g.fn, g.fo), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi);
     s->count();
 }
 
@@ -993,10 +1001,10 @@ static void ph_pp_post(rmt3d_scene *s) {
     const grid_dev &g = s->g;
     size_t nn = (size_t)g.fm * g.fn * g.fo;
     k_mean<<<kMeanBlocks, 256, 0, s->st>>>(s->fem.sol(), nn, 1 / (double)nn, s->d_mean, s->mean_ticket);
-    k_fem_extract<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->dF, s->fem.sol(), s->d_mean);
+    k_fem_extract<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.sol(), s->d_mean);
     s->count(2);
     comm_pressure(s);
-    k_sub_pgrad<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->dF, s->dt, s->d.var_den);
+    k_sub_pgrad<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->dt, s->d.var_den);
     s->count();
 }
 
@@ -1006,9 +1014,9 @@ static void ph_final(rmt3d_scene *s) {
     const grid_dev &g = s->g;
     if (g.n_obj > 0) {
         // update_rho follows in the same pass (var_den)
-        k_refmap_full<<<lin_blocks(g.ncell), 256, 0, s->st>>>(g, s->dF, s->d.var_den);
+        k_refmap_full<<<lin_blocks(g.ncell), 256, 0, s->st>>>(g, s->hF, s->d.var_den);
         s->count();
-        k_redraw<<<lin_blocks(g.ncell), 256, 0, s->st>>>(g, s->dF, s->d.nlayers, s->counters + 4);
+        k_redraw<<<lin_blocks(g.ncell), 256, 0, s->st>>>(g, s->hF, s->d.nlayers, s->counters + 4);
         s->count();
     }
     fill_boundary_cc(s);
@@ -1721,7 +1729,7 @@ static int run_graph(rmt3d_scene *s, int nsteps, int *status) {
 // in a fixed order
 static int div_u(rmt3d_scene *s, double *out) {
     const grid_dev &g = s->g;
-    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->dF, s->fem.rhs(), s->gradphi);
+    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi);
     k_divu_l2<<<kMeanBlocks, 256, 0, s->st>>>(g, s->fem.rhs(), s->d_diag, s->diag_ticket);
     s->count(2);
     CK(cudaMemcpyAsync(s->h_scalar, s->d_diag, sizeof(double), cudaMemcpyDeviceToHost, s->st));
@@ -1939,7 +1947,7 @@ extern "C" int rmt3d_scene_create(const rmt3d_scene_desc *desc, void *stream, rm
     for (int c = 0; c < 9; c++) s->plan(&F.sigma[c], n);
     if (d.var_den) s->plan(&F.rho, n);
     for (int o = 0; o < d.n_obj; o++) {
-        objmap_dev &m = F.om[o];
+        objmap_dev &m = s->hom[o];
         s->plan(&m.code, n), s->plan(&m.code_prev, n);
         for (int c = 0; c < 3; c++)
             s->plan(&m.x[c], n), s->plan(&m.xp[c], n), s->plan(&m.x_prev[c], n), s->plan(&m.det[c], n), s->plan(&m.el[c], n);
@@ -1949,15 +1957,15 @@ extern "C" int rmt3d_scene_create(const rmt3d_scene_desc *desc, void *stream, rm
     if (d.n_obj > 0) {
         const size_t no = (size_t)d.n_obj * n;
         s->plan(&s->lay, no), s->plan(&s->inl, no), s->plan(&s->front[0], no), s->plan(&s->front[1], no);
-        s->plan(&s->fcnt, (size_t)d.nlayers * kMaxObj), s->plan(&s->mlist, n), s->plan(&s->mcnt, 1);
+        s->plan(&s->fcnt, 3 * kMaxObj), s->plan(&s->mlist, n), s->plan(&s->mcnt, 1);
     }
     e |= s->commit_slab();
     for (int o = 0; o < d.n_obj && !e; o++) {
-        cudaMemsetAsync(F.om[o].code, 0xff, n * sizeof(int), s->st);
-        cudaMemsetAsync(F.om[o].code_prev, 0xff, n * sizeof(int), s->st);
+        cudaMemsetAsync(s->hom[o].code, 0xff, n * sizeof(int), s->st);
+        cudaMemsetAsync(s->hom[o].code_prev, 0xff, n * sizeof(int), s->st);
     }
     e |= s->alloc(&s->lx, g.sm4) | s->alloc(&s->ly, g.sn4) | s->alloc(&s->lz, g.so4);
-    e |= s->alloc(&s->dF, 1);
+    e |= s->alloc(&s->dF, 1) | s->alloc(&s->dom, kMaxObj);
     if ((d.run.dump_code & 1) && d.run.ntracers > 0) {
         s->ntr = d.run.ntracers;
         e |= s->alloc(&s->tr_pc, 3 * (size_t)s->ntr) | s->alloc(&s->tr_rp, 6 * (size_t)s->ntr) |
@@ -2012,6 +2020,9 @@ extern "C" int rmt3d_scene_create(const rmt3d_scene_desc *desc, void *stream, rm
     cudaMemcpyAsync(s->lx, s->hlx.data(), g.sm4 * 8, cudaMemcpyHostToDevice, s->st);
     cudaMemcpyAsync(s->ly, s->hly.data(), g.sn4 * 8, cudaMemcpyHostToDevice, s->st);
     cudaMemcpyAsync(s->lz, s->hlz.data(), g.so4 * 8, cudaMemcpyHostToDevice, s->st);
+    F.om = s->dom;
+    for (int o = 0; o < d.n_obj; o++) F.code[o] = s->hom[o].code;
+    cudaMemcpyAsync(s->dom, s->hom, sizeof(s->hom), cudaMemcpyHostToDevice, s->st);
     cudaMemcpyAsync(s->dF, &F, sizeof(F), cudaMemcpyHostToDevice, s->st);
     s->mac.launches = &s->launches;
     s->fem.launches = &s->launches;
@@ -2225,7 +2236,7 @@ extern "C" int rmt3d_init_iter(rmt3d_scene *s) {
         if ((e = init_fluid(s))) return e;
         if ((e = init_refmap(s))) return e;
         if (s->g.n_obj > 0) {
-            k_reset_extraps<<<lin_blocks(s->g.ncell), 256, 0, s->st>>>(s->g, s->dF);
+            k_reset_extraps<<<lin_blocks(s->g.ncell), 256, 0, s->st>>>(s->g, s->hF);
             s->count();
         }
         init_extrapolate(s);
@@ -2341,7 +2352,7 @@ extern "C" int rmt3d_get_scalar(rmt3d_scene *s, int which, double *v) {
             long long cnt = 0;
             std::vector<int> code(s->g.ncell);
             for (int o = 0; o < s->g.n_obj; o++) {
-                CK(copy_sync(s, code.data(), s->hF.om[o].code, s->g.ncell * sizeof(int), cudaMemcpyDeviceToHost));
+                CK(copy_sync(s, code.data(), s->hom[o].code, s->g.ncell * sizeof(int), cudaMemcpyDeviceToHost));
                 for (int c : code) cnt += (c > 0);
             }
             *v = (double)cnt;
@@ -2433,7 +2444,7 @@ extern "C" int rmt3d_get_refmap(rmt3d_scene *s, int obj, int *code, double *x, d
     if (!s) return fail(RMT3D_ERR_INVALID, "null scene");
     if (obj < 0 || obj >= s->g.n_obj) return fail(RMT3D_ERR_INVALID, "object index out of range");
     const size_t n = s->g.ncell;
-    objmap_dev &m = s->hF.om[obj];
+    objmap_dev &m = s->hom[obj];
     CK(cudaStreamSynchronize(s->st));
     if (code) CK(copy_sync(s, code, m.code, n * sizeof(int), cudaMemcpyDeviceToHost));
     for (int c = 0; c < 3; c++) {
@@ -2508,7 +2519,7 @@ extern "C" int rmt3d_import_reference(rmt3d_scene *s, const void *field_aos, con
                 unsigned int cc = *(const unsigned int *)rec;
                 if ((int)(cc & 1023) == o + 1) take(ext_index[q], rec, (cc >> 10) & 63);
             }
-            objmap_dev &m = s->hF.om[o];
+            objmap_dev &m = s->hom[o];
             CK(copy_sync(s, m.code, code.data(), n * sizeof(int), cudaMemcpyHostToDevice));
             for (int c = 0; c < 3; c++) {
                 CK(copy_sync(s, m.x[c], X.data() + c * n, n * 8, cudaMemcpyHostToDevice));
@@ -2561,7 +2572,7 @@ extern "C" int rmt3d_export_reference(rmt3d_scene *s, void *field_aos, void *ref
     std::vector<int> code(n);
     std::vector<double> X(3 * n), XP(3 * n), FX(18 * n), GP(9 * n), DT(3 * n), EL(3 * n);
     for (int o = 0; o < s->g.n_obj; o++) {
-        objmap_dev &m = s->hF.om[o];
+        objmap_dev &m = s->hom[o];
         CK(copy_sync(s, code.data(), m.code, n * sizeof(int), cudaMemcpyDeviceToHost));
         for (int c = 0; c < 3; c++) {
             CK(copy_sync(s, X.data() + c * n, m.x[c], n * 8, cudaMemcpyDeviceToHost));
@@ -2697,12 +2708,39 @@ extern "C" int rmt3d_macro(rmt3d_scene *s, rmt3d_macro_data *out) {
     const grid_dev &g = s->g;
     out->time = s->time;
     out->n_obj = g.n_obj;
-    int e = div_u(s, &out->div_u_l2);
-    if (e) return e;
-    double v[8];
+    // every reduction in turn into the scene's scratch, each copied out behind
+    // it, and one wait for all of them
+    constexpr int kHostVals = 1 + 8 + 7 * RMT3D_MAX_OBJ + kDiagVals;
+    double *h = (double *)pinned_get(kHostVals * sizeof(double));
+    if (!h) return fail(RMT3D_ERR_OOM, "pinned allocation failed");
+    double *const v = h + 1, *const w0 = v + 8, *const d = w0 + 7 * RMT3D_MAX_OBJ;
+    auto fetch = [&](double *dst, int n) {
+        return cudaMemcpyAsync(dst, s->d_diag, n * sizeof(double), cudaMemcpyDeviceToHost, s->st);
+    };
+    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi);
+    k_divu_l2<<<kMeanBlocks, 256, 0, s->st>>>(g, s->fem.rhs(), s->d_diag, s->diag_ticket);
+    cudaError_t ce = fetch(h, 1);
     k_macro_cells<<<kMeanBlocks, 256, 0, s->st>>>(g, s->dF, s->lz, s->d.var_den, s->d_diag, s->diag_ticket);
-    s->count();
-    CK(copy_sync(s, v, s->d_diag, 8 * sizeof(double), cudaMemcpyDeviceToHost));
+    if (ce == cudaSuccess) ce = fetch(v, 8);
+    s->count(3);
+    for (int o = 0; o < g.n_obj; o++) {
+        k_macro_obj<<<kMeanBlocks, 256, 0, s->st>>>(g, s->dF, s->lx, s->ly, s->lz, o, s->d_diag, s->diag_ticket);
+        s->count();
+        if (ce == cudaSuccess) ce = fetch(w0 + 7 * o, 7);
+    }
+    if (g.n_obj > 0) {
+        k_solid_diag<<<kMeanBlocks, 256, 0, s->st>>>(g, s->dF, s->lx, s->ly, s->lz, s->d_diag, s->diag_ticket);
+        s->count();
+        if (ce == cudaSuccess) ce = fetch(d, kDiagVals);
+    }
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s->st);
+    else cudaStreamSynchronize(s->st);
+    struct give_back {
+        double *p;
+        ~give_back() { pinned_put(p, kHostVals * sizeof(double)); }
+    } keep{h};
+    CK(ce);
+    out->div_u_l2 = sqrt(h[0] / ((double)g.fm * g.fn * g.fo));
     // total_momentum: sum * dx * dy * dz; total_energy: each sum * (dx dy dz)
     for (int c = 0; c < 3; c++) out->momentum[c] = v[c] * g.dx * g.dy * g.dz;
     const double dv = g.dx * g.dy * g.dz;
@@ -2714,10 +2752,7 @@ extern "C" int rmt3d_macro(rmt3d_scene *s, rmt3d_macro_data *out) {
     out->div_u_max = v[6];
     out->div_u_min = -v[7];
     for (int o = 0; o < g.n_obj; o++) {
-        double w[7];
-        k_macro_obj<<<kMeanBlocks, 256, 0, s->st>>>(g, s->dF, s->lx, s->ly, s->lz, o, s->d_diag, s->diag_ticket);
-        s->count();
-        CK(copy_sync(s, w, s->d_diag, 7 * sizeof(double), cudaMemcpyDeviceToHost));
+        const double *const w = w0 + 7 * o;
         // sim_manager::compute_avgs: means, 0 for an object without weight
         for (int c = 0; c < 3; c++) {
             out->velocity[o][c] = w[0] != 0. ? w[4 + c] / w[0] : 0.;
@@ -2725,8 +2760,6 @@ extern "C" int rmt3d_macro(rmt3d_scene *s, rmt3d_macro_data *out) {
         }
     }
     if (g.n_obj > 0) {
-        double d[kDiagVals];
-        if ((e = solid_diag(s, d))) return e;
         out->dev_detF = sqrt(d[4] * dv);
         out->max_dev_detF = sqrt(d[5]);
     }
@@ -2763,7 +2796,7 @@ extern "C" int rmt3d_slice(rmt3d_scene *s, int type, int dim, int point, int obj
     }
     const grid_dev &g = s->g;
     if (type == 18) {  // fill_pp_rhs first (fluid_3d_io.cc:162-164)
-        k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->dF, s->fem.rhs(), s->gradphi);
+        k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi);
         s->count();
     }
     double *d = nullptr;
@@ -2924,13 +2957,13 @@ extern "C" size_t rmt3d_scene_footprint(const rmt3d_scene_desc *d) {
     b += (size_t)d->n_obj * (2 * slab_pad(n * sizeof(int)) + 51 * slab_pad(n * sizeof(double)));
     if (d->n_obj > 0) {
         const size_t no = (size_t)d->n_obj * n;
-        b += slab_pad(no * sizeof(uint8_t)) + 3 * slab_pad(no * sizeof(int)) + slab_pad((size_t)d->nlayers * kMaxObj * sizeof(int)) +
+        b += slab_pad(no * sizeof(uint8_t)) + 3 * slab_pad(no * sizeof(int)) + slab_pad(3 * kMaxObj * sizeof(int)) +
              slab_pad(n * sizeof(int)) + slab_pad(sizeof(int));
     }
     if ((d->run.dump_code & 1) && d->run.ntracers > 0)
         b += (size_t)d->run.ntracers * (3 * sizeof(int) + 6 * sizeof(double) + sizeof(uint8_t));
     b += (size_t)(d->sys_size[0] + 4 + d->sys_size[1] + 4 + d->sys_size[2] + 4) * sizeof(double);
-    b += sizeof(fields_dev) + sizeof(scene_ctl) + (1 + kMeanBlocks + 4) * sizeof(double) + sizeof(unsigned);
+    b += sizeof(fields_dev) + kMaxObj * sizeof(objmap_dev) + sizeof(scene_ctl) + (1 + kMeanBlocks + 4) * sizeof(double) + sizeof(unsigned);
     b += kDiagVals * (1 + kMeanBlocks) * sizeof(double) + sizeof(unsigned);
     int prd[3], nm[3], nf[3];
     for (int a = 0; a < 3; a++) {
@@ -3034,12 +3067,12 @@ extern "C" int rmt3d_scene_destroy(rmt3d_scene *s) {
 // ---------------------------------------------------------------------------
 namespace {
 constexpr size_t kNoallocMaxNodes = 65 * 65 * 65;
-constexpr size_t kNoallocHeader = 16384;  // accumulator + argument block, 256-aligned
+constexpr size_t kNoallocHeader = 16384;  // ticket + reduction partials, 256-aligned
 constexpr size_t kNoallocBytes = kNoallocHeader + kNoallocMaxNodes * sizeof(double);
-// [0, 256): reduction ticket; [256, kNoallocRed): argument block;
-// [kNoallocRed, ...): fixed-order reduction partials of k_divu_l2
-constexpr size_t kNoallocRed = 256 + (sizeof(fields_dev) + 255) / 256 * 256;
-static_assert(kNoallocRed + (1 + kMeanBlocks) * sizeof(double) <= kNoallocHeader, "argument block does not fit");
+// [0, 256): reduction ticket; [kNoallocRed, ...): fixed-order reduction
+// partials of k_divu_l2
+constexpr size_t kNoallocRed = 256;
+static_assert(kNoallocRed + (1 + kMeanBlocks) * sizeof(double) <= kNoallocHeader, "partials do not fit");
 }  // namespace
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
@@ -3099,8 +3132,8 @@ extern "C" int rmt3d_div_u_noalloc(const int sys_size[3], const int periodic[3],
         gp.v[i][1] = (2 * ((i / 2) % 2) - 1) * fac;
         gp.v[i][2] = (2 * (i / 4) - 1) * fac;
     }
-    // argument block: only the arrays div_u reads
-    static thread_local fields_dev hf;
+    // only the arrays div_u reads
+    fields_dev hf;
     memset(&hf, 0, sizeof(hf));
     for (int c = 0; c < 3; c++) hf.dvel[c] = const_cast<double *>(dvel[c]);
     for (int f = 0; f < 6; f++)
@@ -3110,12 +3143,10 @@ extern "C" int rmt3d_div_u_noalloc(const int sys_size[3], const int periodic[3],
     if (e) return e;
     cudaStream_t st = (cudaStream_t)stream;
     unsigned *ticket = (unsigned *)base;
-    fields_dev *dF = (fields_dev *)(base + 256);
     double *red = (double *)(base + kNoallocRed);
     double *rhs = (double *)(base + kNoallocHeader);
     CK(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));
-    CK(cudaMemcpyAsync(dF, &hf, sizeof(hf), cudaMemcpyHostToDevice, st));
-    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, st>>>(g, dF, rhs, gp);
+    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, st>>>(g, hf, rhs, gp);
     k_divu_l2<<<kMeanBlocks, 256, 0, st>>>(g, rhs, red, ticket);
     double sum = 0;
     CK(cudaMemcpyAsync(&sum, red, sizeof(double), cudaMemcpyDeviceToHost, st));
