@@ -387,9 +387,10 @@ __device__ __forceinline__ void make_pass(const slab_level &L, int rank, int col
 
 // one colour pass (MODE 0) or the residual of one colour's points (MODE 1)
 template <typename T, int KIND, bool VD, int MODE>
-__device__ __forceinline__ void colour_pass(const slab_ctx<T> &C, const slab_pass &P, const slab_view<T> &V,
+__device__ __forceinline__ void colour_pass(const slab_ctx<T> &C, const slab_pass &table, const slab_view<T> &V,
                                             int colour, int use) {
-    if (C.tid >= P.tot) return;
+    if (C.tid >= table.tot) return;
+    const slab_pass P = table;  // in registers: the stores below could alias it
     if (KIND == 1) {
         for (int t = C.tid; t < P.tot; t += kSlabThreads) {
             if (t < P.tin) {
@@ -441,9 +442,12 @@ __device__ __forceinline__ void smooth_level(const slab_ctx<T> &C, const slab_vi
         const int colour = s % nc;
         if (V.async) {
             uint64_t *bar = C.bar + (use & 1);
-            if (C.tid == 0) halo_arm(bar, P[colour].bytes);
+            // one thread of the last warp, which has the fewest points, waits for
+            // the neighbours; the block barrier hands on what it saw (every
+            // warp polling cost a quarter of a pass's issue slots)
+            if (C.tid == kSlabThreads - 1) halo_arm(bar, P[colour].bytes);
             colour_pass<T, KIND, VD, 0>(C, P[colour], V, colour, use);
-            if (*C.failed == 0 && !halo_wait(bar, (use >> 1) & 1)) *C.failed = 1;
+            if (C.tid == kSlabThreads - 1 && *C.failed == 0 && !halo_wait(bar, (use >> 1) & 1)) *C.failed = 1;
             __syncthreads();
             use++;
         } else {
@@ -710,9 +714,10 @@ __device__ __forceinline__ void slab_cycle(const pmg_args &A, const slab_args &S
                 const int row = fdiv(t, L.inv_w0), ii = t - row * wx;
                 const int kl = fdiv(row, L.inv_w1), jj = row - kl * wy;
                 const int i = wrapi(ii - 1, c0, L.p0), j = wrapi(jj - 1, c1, L.p1), k = wrapi(k0 + kl - 1, c2, L.p2);
-                // a node may have an index past the last cell (walled axis)
-                if (i < 0 || j < 0 || k < 0) continue;
-                C.sm[L.oi + kl * L.PX + jj * L.RS + col(L, ii - 1)] = ri[i + c0 * (j + (size_t)c1 * k)];
+                // (a node may have an index past the last cell of a walled axis)
+                const bool ok = (i | j | k) >= 0;
+                const T v = ri[ok ? i + c0 * (j + (size_t)c1 * k) : 0];
+                C.sm[L.oi + kl * L.PX + jj * L.RS + col(L, ii - 1)] = ok ? v : (T)0;
             }
         }
     cl_barrier();
