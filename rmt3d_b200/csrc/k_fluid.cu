@@ -45,40 +45,50 @@ __global__ void k_periodic_copy(grid_dev g, ptr_list pl, int corner) {
 }
 
 // -------------------------------------------------------------------------
-// Physical BC ghost fill of one face, face_gm::set_ghost_cc
-// (fields.hh:765-800): both ghost layers, the whole tangential extent.
+// Physical BC ghost fill of every wall, face_gm::set_ghost_cc (fields.hh:
+// 765-800): both ghost layers, the whole tangential extent.  The reference
+// fills the axes in order x, y, z, a later axis mirroring the earlier ones'
+// ghost values at edges and corners; each ghost cell here starts from the cell
+// that all its mirrors lead to and applies the axes' rules in that order, so
+// one launch does what three in a chain did.  (Along a periodic axis a ghost
+// cell is not mirrored but read, as the three passes did.)
 // -------------------------------------------------------------------------
-__global__ void k_bc_cc(grid_dev g, int n, bc_face lo, bc_face hi, double *u, double *v, double *w) {
-    // both faces of axis n in one launch: blockIdx.z = 2 * side + layer - 1.
-    // The two faces write disjoint ghost layers and read only cells of their
-    // own side, so they run together; the axes still run in order, x, y, z,
-    // since a later axis reads the earlier axes' ghost values at edges.
-    const int lower = (blockIdx.z < 2);
-    const int face = 2 * n + (lower ? 0 : 1);
-    const bc_face &bc = lower ? lo : hi;
-    const int t0 = (n == 0) ? 1 : 0, t1 = (n == 2) ? 1 : 2;
-    const int ext[3] = {g.sm4, g.sn4, g.so4};
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    int b = blockIdx.y * blockDim.y + threadIdx.y;
-    int layer = (blockIdx.z & 1) + 1;  // 1 or 2
+__global__ void k_bc_cc(grid_dev g, int walls, bc_faces bcs, double *u, double *v, double *w) {
+    // blockIdx.z = 4 * axis + 2 * side + layer - 1
+    const int n = blockIdx.z >> 2, upper = (blockIdx.z >> 1) & 1, layer = (blockIdx.z & 1) + 1;
+    if (!((walls >> n) & 1)) return;
+    const int ext[3] = {g.sm4, g.sn4, g.so4}, len[3] = {g.sm, g.sn, g.so};
+    const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
+    const int t0 = n == 0 ? 1 : 0, t1 = n == 2 ? 1 : 2;
     if (a >= ext[t0] || b >= ext[t1]) return;
-    (void)face;
-    // flat indices from the strides of the three axes (no runtime-indexed
-    // arrays, which would live in local memory)
-    const int sa = t0 == 0 ? 1 : g.sm4, sb = t1 == 1 ? g.sm4 : g.smn4;
-    const int sn_ = n == 0 ? 1 : (n == 1 ? g.sm4 : g.smn4);
-    const int ln = n == 0 ? g.sm : (n == 1 ? g.sn : g.so);
-    const int gn = lower ? 2 - layer : 2 + ln - 1 + layer;
-    const int mn = lower ? 2 + layer - 1 : 2 + ln - layer;
-    const int gi = a * sa + b * sb + gn * sn_;
-    const int mi = a * sa + b * sb + mn * sn_;
-    const double sgn = lower ? -1 : 1;
-    const double dn = 2 * fabs(0.5 * bc.h * (2 * layer - 1));
+    const int gn = upper ? 1 + len[n] + layer : 2 - layer;
+    const int c[3] = {n == 0 ? gn : a, n == 1 ? gn : (n == 0 ? a : b), n == 2 ? gn : b};
+    // the cell belongs to the last wall axis it is a ghost of
+    if (n < 1 && ((walls >> 1) & 1) && (c[1] < 2 || c[1] >= 2 + len[1])) return;
+    if (n < 2 && ((walls >> 2) & 1) && (c[2] < 2 || c[2] >= 2 + len[2])) return;
+    int m[3];
+    bool gh[3], up[3];
+    double dn[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        double *vc = c == 0 ? u : (c == 1 ? v : w);
-        if (bc.bct[c] == 1) vc[gi] = 2 * bc.bcv[c] - vc[mi];
-        else vc[gi] = sgn * dn * bc.bcv[c] + vc[mi];
+    for (int d = 0; d < 3; d++) {
+        up[d] = c[d] >= 2 + len[d];
+        gh[d] = ((walls >> d) & 1) && (c[d] < 2 || up[d]);
+        const int lay = up[d] ? c[d] - 1 - len[d] : 2 - c[d];
+        m[d] = !gh[d] ? c[d] : (up[d] ? 2 + len[d] - lay : 1 + lay);
+        dn[d] = 2 * fabs(0.5 * bcs.f[2 * d].h * (2 * lay - 1));
+    }
+    const int gi = gidx(g, c[0], c[1], c[2]), mi = gidx(g, m[0], m[1], m[2]);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        double *vc = q == 0 ? u : (q == 1 ? v : w);
+        double val = vc[mi];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            if (gh[d]) {
+                const bc_face &bc = bcs.f[2 * d + (up[d] ? 1 : 0)];
+                val = bc.bct[q] == 1 ? 2 * bc.bcv[q] - val : (up[d] ? 1. : -1.) * dn[d] * bc.bcv[q] + val;
+            }
+        vc[gi] = val;
     }
 }
 
@@ -942,11 +952,15 @@ template __global__ void k_upwind<float>(grid_dev, const __grid_constant__ field
 // MAC projection: rhs (fill_mac_rhs, fluid_3d.cc:2244-2265), solution
 // extraction (:2268-2281) and face correction (subtract_q_grad, :2284-2304).
 // -------------------------------------------------------------------------
-__global__ void k_mac_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, double cdt) {
+// time_p: the simulation time, advanced by `half` (the first half of the step
+// ends before this kernel; null: advanced elsewhere)
+__global__ void k_mac_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, double cdt, double *time_p,
+                          double half) {
     const fields_dev *__restrict__ F = &F_;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int j = blockIdx.y * blockDim.y + threadIdx.y;
     int k = blockIdx.z * blockDim.z + threadIdx.z;
+    if (time_p && (i | j | k) == 0) *time_p += half;
     if (i >= g.sm || j >= g.sn || k >= g.so) return;
     const int ind = gidx(g, i + 2, j + 2, k + 2);
     const double fac = g.dx / (2 * cdt);
@@ -955,35 +969,36 @@ __global__ void k_mac_rhs(grid_dev g, const __grid_constant__ fields_dev F_, dou
     r[i + g.sm * (j + g.sn * k)] = s;
 }
 
-__global__ void k_mac_extract(grid_dev g, const __grid_constant__ fields_dev F_, const double *x) {
+// The solution x into q and the correction of the faces, in one pass: a
+// neighbour's value comes from x too, or, beyond a wall, from q's ghost cell,
+// which this kernel leaves alone.
+__global__ void k_sub_qgrad(grid_dev g, const __grid_constant__ fields_dev F_, const double *__restrict__ x, double cdt,
+                            int var_den) {
     const fields_dev *__restrict__ F = &F_;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    int k = blockIdx.z * blockDim.z + threadIdx.z;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z * blockDim.z + threadIdx.z;
     if (i >= g.sm || j >= g.sn || k >= g.so) return;
-    F->q[gidx(g, i + 2, j + 2, k + 2)] = x[i + g.sm * (j + g.sn * k)];
-}
-
-__global__ void k_sub_qgrad(grid_dev g, const __grid_constant__ fields_dev F_, double cdt, int var_den) {
-    const fields_dev *__restrict__ F = &F_;
-    int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-    int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-    int k = blockIdx.z * blockDim.z + threadIdx.z + 2;
-    if (i >= g.sm + 2 || j >= g.sn + 2 || k >= g.so + 2) return;
-    const int ind = gidx(g, i, j, k);
+    const int ind = gidx(g, i + 2, j + 2, k + 2);
     const int strides[3] = {1, g.sm4, g.smn4};
+    const int c[3] = {i, j, k}, len[3] = {g.sm, g.sn, g.so}, xs[3] = {1, g.sm, g.sm * g.sn};
+    const int xi = i + g.sm * (j + g.sn * k);
     const double fac = 2 * cdt * g.dxsp;
-    const double *q = F->q;
+    const double q0 = x[xi];
+    F->q[ind] = q0;
     for (int f = 0; f < 3; f++) {
-        int s = strides[f];
+        const int s = strides[f];
+        const bool lo = c[f] > 0 || g.prd[f], hi = c[f] < len[f] - 1 || g.prd[f];
+        const double ql = lo ? x[xi + (c[f] > 0 ? -xs[f] : (len[f] - 1) * xs[f])] : F->q[ind - s];
+        const double qh = hi ? x[xi + (c[f] < len[f] - 1 ? xs[f] : (1 - len[f]) * xs[f])] : F->q[ind + s];
         double down, up;
         if (var_den) {
             const double *rho = F->rho;
-            down = fac * (q[ind] - q[ind - s]) / (0.5 * (rho[ind] + rho[ind - s]));
-            up = fac * (q[ind + s] - q[ind]) / (0.5 * (rho[ind + s] + rho[ind]));
+            down = fac * (q0 - ql) / (0.5 * (rho[ind] + rho[ind - s]));
+            up = fac * (qh - q0) / (0.5 * (rho[ind + s] + rho[ind]));
         } else {
-            down = fac * (q[ind] - q[ind - s]);
-            up = fac * (q[ind + s] - q[ind]);
+            down = fac * (q0 - ql);
+            up = fac * (qh - q0);
         }
         face_st(g, F, 3 * (2 * f) + f, ind, face_ld(g, F, 3 * (2 * f) + f, ind) - down);
         face_st(g, F, 3 * (2 * f + 1) + f, ind, face_ld(g, F, 3 * (2 * f + 1) + f, ind) - up);
@@ -1055,11 +1070,14 @@ __device__ inline bool elem_in_domain(const grid_dev &g, int ei, int ej, int ek)
            (g.prd[2] || (ek >= 0 && ek <= g.so - 1));
 }
 
-__global__ void k_fem_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, gradphi_t gp) {
+// time_p as in k_mac_rhs, for the second half of the step
+__global__ void k_fem_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, gradphi_t gp, double *time_p,
+                          double half) {
     const fields_dev *__restrict__ F = &F_;
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     int b = blockIdx.y * blockDim.y + threadIdx.y;
     int c = blockIdx.z * blockDim.z + threadIdx.z;
+    if (time_p && (a | b | c) == 0) *time_p += half;
     if (a >= g.fm || b >= g.fn || c >= g.fo) return;
     double s = 0;
     // element (ei,ej,ek) touches node (a,b,c) as local node (a-ei)+2(b-ej)+4(c-ek)
@@ -1117,31 +1135,28 @@ __global__ void k_fem_rhs(grid_dev g, const __grid_constant__ fields_dev F_, dou
     r[a + g.fm * (b + g.fn * c)] = s;
 }
 
-// p += x - mean, dp = x - mean over FEM nodes (extract_pp_soln, :2685-2712)
-__global__ void k_fem_extract(grid_dev g, const __grid_constant__ fields_dev F_, const double *x, const double *mean) {
+// p += x - mean, dp = x - mean over the FEM nodes (extract_pp_soln,
+// fluid_3d.cc:2685-2712), and for the cell above each node u, dvel -= dt
+// grad(dp) (subtract_pres_grad, :2717-2753, with neg_pres_dgrad), whose eight
+// nodal values come from x too.
+__global__ void k_sub_pgrad(grid_dev g, const __grid_constant__ fields_dev F_, const double *__restrict__ x,
+                            const double *mean, double dt, int var_den) {
     const fields_dev *__restrict__ F = &F_;
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    int b = blockIdx.y * blockDim.y + threadIdx.y;
-    int c = blockIdx.z * blockDim.z + threadIdx.z;
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = blockIdx.y * blockDim.y + threadIdx.y;
+    const int c = blockIdx.z * blockDim.z + threadIdx.z;
     if (a >= g.fm || b >= g.fn || c >= g.fo) return;
     const double m = *mean;
-    const double v = x[a + g.fm * (b + g.fn * c)];
     const int ind = gidx(g, a + 2, b + 2, c + 2);
-    F->p[ind] += (v - m);
-    F->dp[ind] = (v - m);
-}
-
-// u, dvel -= dt grad(dp), subtract_pres_grad (:2717-2753) with neg_pres_dgrad
-__global__ void k_sub_pgrad(grid_dev g, const __grid_constant__ fields_dev F_, double dt, int var_den) {
-    const fields_dev *__restrict__ F = &F_;
-    int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-    int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-    int k = blockIdx.z * blockDim.z + threadIdx.z + 2;
-    if (i >= g.sm + 2 || j >= g.sn + 2 || k >= g.so + 2) return;
-    const int ind = gidx(g, i, j, k);
-    const int s1 = g.sm4, s2 = g.smn4;
+    // the next node along an axis, round the seam of a periodic one
+    const int na = a + 1 < g.fm ? a + 1 : 0, nb = b + 1 < g.fn ? b + 1 : 0, nc = c + 1 < g.fo ? c + 1 : 0;
     double pr[8];
-    for (int n = 0; n < 8; n++) pr[n] = F->dp[ind + n % 2 + s1 * ((n / 2) % 2) + (n / 4) * s2];
+#pragma unroll
+    for (int n = 0; n < 8; n++)
+        pr[n] = x[(n & 1 ? na : a) + g.fm * ((n & 2 ? nb : b) + g.fn * (n & 4 ? nc : c))] - m;
+    F->p[ind] += pr[0];
+    F->dp[ind] = pr[0];
+    if (a >= g.sm || b >= g.sn || c >= g.so) return;
     double xa = 0, ya = 0, za = 0;
     for (int n = 0; n < 4; n++) {
         xa += pr[2 * n + 1] - pr[2 * n];
@@ -1153,11 +1168,11 @@ __global__ void k_sub_pgrad(grid_dev g, const __grid_constant__ fields_dev F_, d
     ya *= -0.25 * g.dysp;
     za *= -0.25 * g.dzsp;
     double npg[3] = {xa, ya, za};
-    for (int c = 0; c < 3; c++) {
-        if (var_den) npg[c] *= dt / F->rho[ind];
-        else npg[c] *= dt;
-        F->vel[c][ind] += npg[c];
-        F->dvel[c][ind] += npg[c];
+    for (int q = 0; q < 3; q++) {
+        if (var_den) npg[q] *= dt / F->rho[ind];
+        else npg[q] *= dt;
+        F->vel[q][ind] += npg[q];
+        F->dvel[q][ind] += npg[q];
     }
 }
 

@@ -44,7 +44,7 @@ struct gradphi_t {
 };
 
 __global__ void k_periodic_copy(grid_dev g, ptr_list pl, int corner);
-__global__ void k_bc_cc(grid_dev g, int n, bc_face lo, bc_face hi, double *u, double *v, double *w);
+__global__ void k_bc_cc(grid_dev g, int walls, bc_faces bcs, double *u, double *v, double *w);
 __global__ void k_bc_cf(grid_dev g, int walls, bc_faces bcs, const __grid_constant__ fields_dev F_);
 __global__ void k_stress(grid_dev g, const __grid_constant__ fields_dev F_, const int *list, const int *cnt);
 __global__ void k_stress_fluid(grid_dev g, const __grid_constant__ fields_dev F_, int *list, int *cnt);
@@ -59,15 +59,17 @@ void launch_edge_vel_tma(const grid_dev &g, const fields_dev &F, const CUtensorM
                          cudaStream_t st);
 template <typename FT>
 __global__ void k_upwind(grid_dev g, const __grid_constant__ fields_dev F_);
-__global__ void k_mac_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, double cdt);
-__global__ void k_mac_extract(grid_dev g, const __grid_constant__ fields_dev F_, const double *x);
-__global__ void k_sub_qgrad(grid_dev g, const __grid_constant__ fields_dev F_, double cdt, int var_den);
+__global__ void k_mac_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, double cdt, double *time_p,
+                          double half);
+__global__ void k_sub_qgrad(grid_dev g, const __grid_constant__ fields_dev F_, const double *__restrict__ x, double cdt,
+                            int var_den);
 template <typename FT>
 __global__ void k_ustar(grid_dev g, const __grid_constant__ fields_dev F_, const double *lx, const double *ly,
                         const double *lz, double cdt, const double *time_p, int var_den);
-__global__ void k_fem_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, gradphi_t gp);
-__global__ void k_fem_extract(grid_dev g, const __grid_constant__ fields_dev F_, const double *x, const double *mean);
-__global__ void k_sub_pgrad(grid_dev g, const __grid_constant__ fields_dev F_, double dt, int var_den);
+__global__ void k_fem_rhs(grid_dev g, const __grid_constant__ fields_dev F_, double *r, gradphi_t gp, double *time_p,
+                          double half);
+__global__ void k_sub_pgrad(grid_dev g, const __grid_constant__ fields_dev F_, const double *__restrict__ x,
+                            const double *mean, double dt, int var_den);
 __global__ void k_chk_pack(grid_dev g, const fields_dev *__restrict__ F, double *__restrict__ buf);
 __global__ void k_macro_cells(grid_dev g, const fields_dev *__restrict__ F, const double *lz, int var_den,
                               double *out, unsigned *ticket);

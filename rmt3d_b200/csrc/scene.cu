@@ -174,6 +174,7 @@ struct rmt3d_scene {
     cudaGraphExec_t step_exec = nullptr;
     bool graph_dirty = true;
     bool capturing = false;
+    bool half_due = false;  // a half step of time to be added by the next kernel that can
     bool use_graph = true;
     long long graph_fixed = 0;  // kernels per step outside the multigrid loops
     long long param_version = 0;  // bumped whenever captured step parameters change
@@ -317,13 +318,16 @@ static void periodic(rmt3d_scene *s, std::initializer_list<double *> arrs, std::
 // fill_boundary_cc: set_bc_cc then communicate<1> (fluid_3d.cc:145-152)
 static void fill_boundary_cc(rmt3d_scene *s) {
     const grid_dev &g = s->g;
-    const int ext[3] = {g.sm4, g.sn4, g.so4};
-    for (int n = 0; n < 3; n++) {  // walls come in pairs: both faces of an axis at once
-        if (!s->wall[2 * n]) continue;
-        int t0 = (n == 0) ? 1 : 0, t1 = (n == 2) ? 1 : 2;
-        dim3 gr((ext[t0] + 31) / 32, (ext[t1] + 7) / 8, 4);
-        k_bc_cc<<<gr, dim3(32, 8, 1), 0, s->st>>>(g, n, s->faces[2 * n], s->faces[2 * n + 1], s->hF.vel[0],
-                                                  s->hF.vel[1], s->hF.vel[2]);
+    int walls = 0;  // per axis: walls come in pairs
+    bc_faces bcs;
+    for (int f = 0; f < 6; f++) {
+        bcs.f[f] = s->faces[f];
+        if (s->wall[f]) walls |= 1 << (f / 2);
+    }
+    if (walls) {
+        const int ma = std::max(g.sm4, g.sn4), mb = std::max(g.sn4, g.so4);
+        k_bc_cc<<<dim3((ma + 31) / 32, (mb + 7) / 8, 12), dim3(32, 8, 1), 0, s->st>>>(g, walls, bcs, s->hF.vel[0],
+                                                                                       s->hF.vel[1], s->hF.vel[2]);
         s->count();
     }
     periodic(s, {s->hF.vel[0], s->hF.vel[1], s->hF.vel[2]}, {}, 0);
@@ -838,12 +842,26 @@ static void set_time(rmt3d_scene *s, double t) {
 }
 
 // time += dt/2 (the two halves of fluid_3d::step_forward, fluid_3d.cc:456,
-// :541); the host mirror follows in eager mode and is read back after a
-// graph step
+// :541); the host mirror follows in eager mode and is read back after a graph
+// step.  On the device the next right-hand side's kernel adds it (nothing in
+// between reads the time), a launch fewer; a step that stops before that
+// kernel adds it with flush_half.
 static void advance_half(rmt3d_scene *s) {
     if (!s->capturing) s->time += 0.5 * s->dt;
+    s->half_due = true;
+}
+static void flush_half(rmt3d_scene *s) {
+    if (!s->half_due) return;
+    s->half_due = false;
     k_time_add<<<1, 1, 0, s->st>>>(s->ctl, 0.5 * s->dt);
     s->count();
+}
+
+// the time for the kernel that adds a due half step, else null
+static double *due_time(rmt3d_scene *s) {
+    if (!s->half_due) return nullptr;
+    s->half_due = false;
+    return &s->ctl->time;
 }
 
 // ---- phases of fluid_3d::step_forward (fluid_3d.cc:429-577) ----------------
@@ -885,17 +903,17 @@ static void ph_upwind(rmt3d_scene *s) {
 static void ph_mac_pre(rmt3d_scene *s, double cdt) {
     const grid_dev &g = s->g;
     update_rinv(s);
-    k_mac_rhs<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->mac.rhs(), cdt);
+    k_mac_rhs<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->mac.rhs(), cdt, due_time(s),
+                                                                                            0.5 * s->dt);
     s->count();
 }
 
 static void ph_mac_post(rmt3d_scene *s, double cdt) {
     const grid_dev &g = s->g;
-    k_mac_extract<<<grd(g.sm, g.sn, g.so), blk(), 0, s->st>>>(g, s->hF, s->mac.sol());
+    k_sub_qgrad<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->mac.sol(), cdt,
+                                                                                     s->d.var_den);
     s->count();
     comm_pressure(s);
-    k_sub_qgrad<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, cdt, s->d.var_den);
-    s->count();
     fill_boundary_cf(s);
 }
 
@@ -993,7 +1011,8 @@ static void ph_pp_pre(rmt3d_scene *s) {
     // the density is already that of the current maps: update_rho ran after
     // the reference-map update, and nothing since has moved a map
     update_rinv(s);
-    k_fem_rhs<<<grd_of(s->bshape, g.fm, g.fn, g.fo), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi);
+    k_fem_rhs<<<grd_of(s->bshape, g.fm, g.fn, g.fo), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi,
+                                                                                     due_time(s), 0.5 * s->dt);
     s->count();
 }
 
@@ -1001,11 +1020,10 @@ static void ph_pp_post(rmt3d_scene *s) {
     const grid_dev &g = s->g;
     size_t nn = (size_t)g.fm * g.fn * g.fo;
     k_mean<<<kMeanBlocks, 256, 0, s->st>>>(s->fem.sol(), nn, 1 / (double)nn, s->d_mean, s->mean_ticket);
-    k_fem_extract<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.sol(), s->d_mean);
+    k_sub_pgrad<<<grd_of(s->bshape, g.fm, g.fn, g.fo), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->fem.sol(),
+                                                                                     s->d_mean, s->dt, s->d.var_den);
     s->count(2);
     comm_pressure(s);
-    k_sub_pgrad<<<grd_of(s->bshape, g.sm, g.sn, g.so), blk_of(s->bshape), 0, s->st>>>(g, s->hF, s->dt, s->d.var_den);
-    s->count();
 }
 
 // update_reference_map_full, update_rho, redraw_boundary, boundary fills
@@ -1141,12 +1159,16 @@ static int step_forward(rmt3d_scene *s, int debug, int stop = 99) {
     ph_edges(s);
     if (s->edge_tma) {
         int e = read_ctl(s);
+        if (e || s->h_counters[7] > 0) flush_half(s);
         if (e) return e;
         if (s->h_counters[7] > 0) return fail(RMT3D_ERR_CUDA, "k_edge_vel_tma: a staged velocity plane never arrived");
     }
-    if (stop <= 2) return RMT3D_OK;
+    if (stop <= 3) {
+        if (stop == 3) ph_upwind(s);
+        flush_half(s);
+        return RMT3D_OK;
+    }
     ph_upwind(s);
-    if (stop <= 3) return RMT3D_OK;
     ph_mac_pre(s, s->dt);
     double res = s->mac.run(s->st);
     if (std::isnan(res)) {
@@ -1169,7 +1191,10 @@ static int step_forward(rmt3d_scene *s, int debug, int stop = 99) {
     compute_stress(s);
     if (stop <= 6) return RMT3D_OK;
     ph_ustar(s);
-    if (stop <= 7) return RMT3D_OK;
+    if (stop <= 7) {
+        flush_half(s);
+        return RMT3D_OK;
+    }
     ph_pp_pre(s);
     res = s->fem.run(s->st);
     if (std::isnan(res)) return RMT3D_PROJECTION_ERR;
@@ -1729,7 +1754,7 @@ static int run_graph(rmt3d_scene *s, int nsteps, int *status) {
 // in a fixed order
 static int div_u(rmt3d_scene *s, double *out) {
     const grid_dev &g = s->g;
-    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi);
+    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi, nullptr, 0);
     k_divu_l2<<<kMeanBlocks, 256, 0, s->st>>>(g, s->fem.rhs(), s->d_diag, s->diag_ticket);
     s->count(2);
     CK(cudaMemcpyAsync(s->h_scalar, s->d_diag, sizeof(double), cudaMemcpyDeviceToHost, s->st));
@@ -2717,7 +2742,7 @@ extern "C" int rmt3d_macro(rmt3d_scene *s, rmt3d_macro_data *out) {
     auto fetch = [&](double *dst, int n) {
         return cudaMemcpyAsync(dst, s->d_diag, n * sizeof(double), cudaMemcpyDeviceToHost, s->st);
     };
-    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi);
+    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi, nullptr, 0);
     k_divu_l2<<<kMeanBlocks, 256, 0, s->st>>>(g, s->fem.rhs(), s->d_diag, s->diag_ticket);
     cudaError_t ce = fetch(h, 1);
     k_macro_cells<<<kMeanBlocks, 256, 0, s->st>>>(g, s->dF, s->lz, s->d.var_den, s->d_diag, s->diag_ticket);
@@ -2796,7 +2821,7 @@ extern "C" int rmt3d_slice(rmt3d_scene *s, int type, int dim, int point, int obj
     }
     const grid_dev &g = s->g;
     if (type == 18) {  // fill_pp_rhs first (fluid_3d_io.cc:162-164)
-        k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi);
+        k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, s->st>>>(g, s->hF, s->fem.rhs(), s->gradphi, nullptr, 0);
         s->count();
     }
     double *d = nullptr;
@@ -3146,7 +3171,7 @@ extern "C" int rmt3d_div_u_noalloc(const int sys_size[3], const int periodic[3],
     double *red = (double *)(base + kNoallocRed);
     double *rhs = (double *)(base + kNoallocHeader);
     CK(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));
-    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, st>>>(g, hf, rhs, gp);
+    k_fem_rhs<<<grd(g.fm, g.fn, g.fo), blk(), 0, st>>>(g, hf, rhs, gp, nullptr, 0);
     k_divu_l2<<<kMeanBlocks, 256, 0, st>>>(g, rhs, red, ticket);
     double sum = 0;
     CK(cudaMemcpyAsync(&sum, red, sizeof(double), cudaMemcpyDeviceToHost, st));
