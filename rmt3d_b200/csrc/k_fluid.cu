@@ -1079,20 +1079,34 @@ __global__ void k_fem_rhs(grid_dev g, const __grid_constant__ fields_dev F_, dou
     int c = blockIdx.z * blockDim.z + threadIdx.z;
     if (time_p && (a | b | c) == 0) *time_p += half;
     if (a >= g.fm || b >= g.fn || c >= g.fo) return;
+    // element (ei,ej,ek) touches node (a,b,c) as local node (a-ei)+2(b-ej)+4(c-ek).
+    // The eight elements' increments are loaded together (outside the domain
+    // they lie in the ghost frame); an element that does not exist adds zero.
+    // (Element by element behind its conditions it was a chain of load rounds:
+    // 158 us at 192^3, 28 us at 96^3, and the DRAM time of 192^3 is 35 us.)
     double s = 0;
-    // element (ei,ej,ek) touches node (a,b,c) as local node (a-ei)+2(b-ej)+4(c-ek)
-    for (int ek = c - 1; ek <= c; ek++)
-        for (int ej = b - 1; ej <= b; ej++)
-            for (int ei = a - 1; ei <= a; ei++) {
-                if (ei < -1 || ej < -1 || ek < -1) continue;
-                if (ei > g.fm - 1 || ej > g.fn - 1 || ek > g.fo - 1) continue;
-                if (!elem_in_domain(g, ei, ej, ek)) continue;
-                const int n = (a - ei) + 2 * (b - ej) + 4 * (c - ek);
-                const int ind = gidx(g, ei + 2, ej + 2, ek + 2);
+    const bool ex[2] = {g.prd[0] || a > 0, g.prd[0] || a < g.sm}, ey[2] = {g.prd[1] || b > 0, g.prd[1] || b < g.sn},
+               ez[2] = {g.prd[2] || c > 0, g.prd[2] || c < g.so};
+    const int i8 = gidx(g, a + 1, b + 1, c + 1);
+#pragma unroll
+    for (int dk = 0; dk < 2; dk++)
+#pragma unroll
+        for (int dj = 0; dj < 2; dj++)
+#pragma unroll
+            for (int di = 0; di < 2; di++) {
+                const int n = (1 - di) + 2 * (1 - dj) + 4 * (1 - dk);
+                const int ind = i8 + di + dj * g.sm4 + dk * g.smn4;
                 double val = 0;
+#pragma unroll
                 for (int l = 0; l < 3; l++) val += F->dvel[l][ind] * gp.v[n][l];
-                s += val;
+                s += ex[di] && ey[dj] && ez[dk] ? val : 0.;
             }
+    // most nodes lie on no wall
+    if ((g.prd[0] || (a > 0 && a < g.fm - 1)) && (g.prd[1] || (b > 0 && b < g.fn - 1)) &&
+        (g.prd[2] || (c > 0 && c < g.fo - 1))) {
+        r[a + g.fm * (b + g.fn * c)] = s;
+        return;
+    }
     // domain-face flux terms of non-periodic faces (fluid_3d.cc:2585-2645)
     const int node[3] = {a, b, c};
     const int fdim[3] = {g.fm, g.fn, g.fo};
