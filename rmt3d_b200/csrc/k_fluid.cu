@@ -15,33 +15,21 @@ namespace rmt3d {
 // Periodic ghost copy: replaces fluid_3d::communicate<flags> on one rank
 // (fluid_3d_comm.cc:76-198), where each ghost region whose direction has only
 // periodic components receives the interior slab from the opposite side.
-// corner != 0 selects the nodal table (fluid_3d_comm.cc:55-58), whose extent
-// along a non-periodic axis is one node longer.
+// corner != 0 selects the nodal table (shell_cell).
 // -------------------------------------------------------------------------
-__global__ void k_periodic_copy(grid_dev g, ptr_list pl, int corner) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    int k = blockIdx.z * blockDim.z + threadIdx.z;
-    if (i >= g.sm4 || j >= g.sn4 || k >= g.so4) return;
-    const int c[3] = {i, j, k};
-    const int s[3] = {g.sm, g.sn, g.so};
-    int src[3];
-    bool ghost = false;
-    for (int d = 0; d < 3; d++) {
-        int len = s[d] + ((corner && !g.prd[d]) ? 1 : 0);
-        if (c[d] >= 2 && c[d] < 2 + len) {
-            src[d] = c[d];
-            continue;
-        }
-        if (!g.prd[d]) return;  // wall ghost: not filled by the exchange
-        ghost = true;
-        src[d] = (c[d] < 2) ? c[d] + s[d] : c[d] - s[d];
+// blockIdx.y: the array (one array after another in a thread was a chain of
+// loads and stores)
+__global__ void k_periodic_copy(grid_dev g, ptr_list pl, int corner, int cells) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    int dst, from, a = blockIdx.y;
+    if (t >= cells || !shell_cell(g, corner, t, dst, from)) return;
+    if (a < pl.n) {
+        pl.p[a][dst] = pl.p[a][from];
+        return;
     }
-    if (!ghost) return;
-    int dst = gidx(g, i, j, k), from = gidx(g, src[0], src[1], src[2]);
-    for (int a = 0; a < pl.n; a++) pl.p[a][dst] = pl.p[a][from];
-    for (int a = 0; a < pl.nf; a++) pl.fp[a][dst] = pl.fp[a][from];
-    for (int a = 0; a < pl.ni; a++) pl.ip[a][dst] = pl.ip[a][from];
+    a -= pl.n;
+    if (a < pl.nf) pl.fp[a][dst] = pl.fp[a][from];
+    else pl.ip[a - pl.nf][dst] = pl.ip[a - pl.nf][from];
 }
 
 // -------------------------------------------------------------------------

@@ -242,17 +242,9 @@ __device__ inline void push_layer(const grid_dev &g, const int *front, const int
 // image-backed ghost cells take their image's tag and join its layer
 // (periodic domains only)
 __global__ void k_lay_ghost(grid_dev g, uint8_t *lay, int *inl, int next, int *nfront, int *ncnt) {
-    int ind = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ind >= g.ncell) return;
-    int k = ind / g.smn4, j = (ind % g.smn4) / g.sm4, i = ind % g.sm4;
-    if (!image_backed(g, i, j, k)) return;
-    const int s[3] = {g.sm, g.sn, g.so};
-    int c[3] = {i, j, k};
-    for (int d = 0; d < 3; d++) {
-        if (c[d] < 2) c[d] += s[d];
-        else if (c[d] >= 2 + s[d]) c[d] -= s[d];
-    }
-    const int src = gidx(g, c[0], c[1], c[2]);
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    int ind, src;
+    if (q >= shell_cells(g, 0) || !shell_cell(g, 0, q, ind, src)) return;
     for (int o = 0; o < g.n_obj; o++) {
         const size_t off = (size_t)o * g.ncell;
         uint8_t v = lay[off + src];
@@ -670,17 +662,9 @@ template __global__ void k_extrap_layer<32>(grid_dev, const __grid_constant__ fi
 // domains only).
 __global__ void k_layer_ghost_copy(grid_dev g, const __grid_constant__ fields_dev F_, int L) {
     const fields_dev *__restrict__ F = &F_;
-    int ind = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ind >= g.ncell) return;
-    int k = ind / g.smn4, j = (ind % g.smn4) / g.sm4, i = ind % g.sm4;
-    if (!image_backed(g, i, j, k)) return;
-    const int s[3] = {g.sm, g.sn, g.so};
-    int c[3] = {i, j, k};
-    for (int d = 0; d < 3; d++) {
-        if (c[d] < 2) c[d] += s[d];
-        else if (c[d] >= 2 + s[d]) c[d] -= s[d];
-    }
-    const int src = gidx(g, c[0], c[1], c[2]);
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    int ind, src;
+    if (q >= shell_cells(g, 0) || !shell_cell(g, 0, q, ind, src)) return;
     for (int o = 0; o < g.n_obj; o++) {
         const objmap_dev &m = F->om[o];
         if (m.code[src] != L) continue;

@@ -43,7 +43,7 @@ struct gradphi_t {
     double v[8][3];
 };
 
-__global__ void k_periodic_copy(grid_dev g, ptr_list pl, int corner);
+__global__ void k_periodic_copy(grid_dev g, ptr_list pl, int corner, int cells);
 __global__ void k_bc_cc(grid_dev g, int walls, bc_faces bcs, double *u, double *v, double *w);
 __global__ void k_bc_cf(grid_dev g, int walls, bc_faces bcs, const __grid_constant__ fields_dev F_);
 __global__ void k_stress(grid_dev g, const __grid_constant__ fields_dev F_, const int *list, const int *cnt);

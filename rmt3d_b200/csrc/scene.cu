@@ -302,6 +302,11 @@ static int faces_from_host(rmt3d_scene *s, int c, const double *src) {
 // ---------------------------------------------------------------------------
 // ghost-frame helpers
 // ---------------------------------------------------------------------------
+static void copy_images(rmt3d_scene *s, const ptr_list &pl, int corner) {
+    const int cells = shell_cells(s->g, corner);
+    k_periodic_copy<<<dim3((cells + 255) / 256, pl.n + pl.nf + pl.ni), 256, 0, s->st>>>(s->g, pl, corner, cells);
+}
+
 static void periodic(rmt3d_scene *s, std::initializer_list<double *> arrs, std::initializer_list<int *> iarrs,
                      int corner) {
     if (!(s->g.prd[0] || s->g.prd[1] || s->g.prd[2])) return;
@@ -311,7 +316,7 @@ static void periodic(rmt3d_scene *s, std::initializer_list<double *> arrs, std::
     pl.nf = 0;
     for (double *a : arrs) pl.p[pl.n++] = a;
     for (int *a : iarrs) pl.ip[pl.ni++] = a;
-    k_periodic_copy<<<grd(s->g.sm4, s->g.sn4, s->g.so4), blk(), 0, s->st>>>(s->g, pl, corner);
+    copy_images(s, pl, corner);
     s->count();
 }
 
@@ -357,7 +362,7 @@ static void fill_boundary_cf(rmt3d_scene *s) {
             pl.p[a] = s->hF.fvel[a];
             pl.fp[a] = s->hF.fvel32[a];
         }
-        k_periodic_copy<<<grd(g.sm4, g.sn4, g.so4), blk(), 0, s->st>>>(g, pl, 0);
+        copy_images(s, pl, 0);
         s->count();
     }
 }
@@ -377,7 +382,7 @@ static void comm_face_maps(rmt3d_scene *s) {
         pl.ni = 0;
         pl.nf = 0;
         for (int a = 0; a < 18; a++) pl.p[a] = s->hom[o].fx[a];
-        k_periodic_copy<<<grd(g.sm4, g.sn4, g.so4), blk(), 0, s->st>>>(g, pl, 0);
+        copy_images(s, pl, 0);
         s->count();
     }
 }
@@ -395,7 +400,7 @@ static void comm_primary(rmt3d_scene *s) {
         for (int a = 0; a < 3; a++) pl.p[pl.n++] = m.xp[a];
         pl.ni = 1;
         pl.ip[0] = m.code;
-        k_periodic_copy<<<grd(g.sm4, g.sn4, g.so4), blk(), 0, s->st>>>(g, pl, 0);
+        copy_images(s, pl, 0);
         s->count();
     }
 }
@@ -413,6 +418,7 @@ static void extrapolate(rmt3d_scene *s, bool lay_ready = false) {
     // without a periodic axis no ghost cell is the image of an interior
     // cell, and the two ghost-copy kernels would find nothing to do
     const bool prd = g.prd[0] || g.prd[1] || g.prd[2];
+    const int ng = prd ? lin_blocks(shell_cells(g, 0)) : 0;
     // the list lengths of the layer being fitted, of the one being listed, and
     // of the one after, which the launch zeroes
     auto cnt = [&](int layer) { return s->fcnt + (layer % 3) * kMaxObj; };
@@ -424,7 +430,7 @@ static void extrapolate(rmt3d_scene *s, bool lay_ready = false) {
     k_lay_push<<<nb, 256, 0, s->st>>>(g, s->lay, s->inl, s->front[0], cnt(1));
     s->count();
     if (prd) {
-        k_lay_ghost<<<nb, 256, 0, s->st>>>(g, s->lay, s->inl, 1, s->front[0], cnt(1));
+        k_lay_ghost<<<ng, 256, 0, s->st>>>(g, s->lay, s->inl, 1, s->front[0], cnt(1));
         s->count();
     }
     int cur = 0;
@@ -439,11 +445,11 @@ static void extrapolate(rmt3d_scene *s, bool lay_ready = false) {
                                                          cnt(L + 1), cnt(L + 2));
         s->count();
         if (prd) {
-            k_layer_ghost_copy<<<nb, 256, 0, s->st>>>(g, s->hF, L);
+            k_layer_ghost_copy<<<ng, 256, 0, s->st>>>(g, s->hF, L);
             s->count();
         }
         if (more && prd) {
-            k_lay_ghost<<<nb, 256, 0, s->st>>>(g, s->lay, s->inl, L + 1, s->front[cur ^ 1], cnt(L + 1));
+            k_lay_ghost<<<ng, 256, 0, s->st>>>(g, s->lay, s->inl, L + 1, s->front[cur ^ 1], cnt(L + 1));
             s->count();
         }
         cur ^= 1;
