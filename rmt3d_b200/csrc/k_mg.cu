@@ -43,34 +43,34 @@ __global__ void __launch_bounds__(256) k_mac_rb(lvl_dev L, T *__restrict__ x, co
                                                 const T *__restrict__ ri, unsigned inv) {
     body_mac_rb<T>(L, x, r, colour, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
-template <typename T>
-__global__ void __launch_bounds__(256) k_fem_gs(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour,
-                                                const T *__restrict__ ri, unsigned inv) {
-    body_fem_gs<T>(L, x, r, colour, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
+template <typename T, bool MARCH>
+__global__ void __launch_bounds__(256) k_fem_gs(lvl_dev L, T *x, const T *__restrict__ r, int colour,
+                                                const T *__restrict__ ri, unsigned inv, int pz) {
+    body_fem_gs<T, MARCH>(L, x, r, colour, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y, pz);
 }
-template <typename T, int KIND>
+template <typename T, int KIND, bool MARCH>
 __global__ void __launch_bounds__(256) k_resid(lvl_dev L, const T *__restrict__ x, const T *__restrict__ r,
-                                               T *__restrict__ res, const T *__restrict__ ri, unsigned inv) {
-    body_resid<T, KIND>(L, x, r, res, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
+                                               T *__restrict__ res, const T *__restrict__ ri, unsigned inv, int pz) {
+    body_resid<T, KIND, MARCH>(L, x, r, res, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y, pz);
 }
 // the control's max-norm residual, computed only when the control will read it
-template <int KIND>
+template <int KIND, bool MARCH>
 __global__ void __launch_bounds__(256) k_resid_ctl(lvl_dev L, const double *__restrict__ x,
                                                    const double *__restrict__ r, unsigned long long *mx,
-                                                   const double *__restrict__ ri, const mg_ctl *c, unsigned inv) {
+                                                   const double *__restrict__ ri, const mg_ctl *c, unsigned inv, int pz) {
     if (!c->need_res) return;
-    block_max_into(body_resid_max<KIND>(L, x, r, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y), mx);
+    block_max_into(body_resid_max<KIND, MARCH>(L, x, r, ri, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y, pz), mx);
 }
 template <typename T>
 __global__ void k_mac_restrict(lvl_dev F, lvl_dev C, const T *__restrict__ res, T *__restrict__ rc,
                                T *__restrict__ xc0) {
     body_mac_restrict<T>(F, C, res, rc, xc0, blockIdx.x, blockIdx.y, blockIdx.z);
 }
-template <int KIND>
+template <int KIND, bool MARCH>
 __global__ void __launch_bounds__(256) k_resid_to_f32(lvl_dev L, const double *__restrict__ x,
                                                       const double *__restrict__ r, const double *__restrict__ ri,
-                                                      float *__restrict__ rs, float *__restrict__ xs, unsigned inv) {
-    body_resid_to_f32<KIND>(L, x, r, ri, rs, xs, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
+                                                      float *__restrict__ rs, float *__restrict__ xs, unsigned inv, int pz) {
+    body_resid_to_f32<KIND, MARCH>(L, x, r, ri, rs, xs, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y, pz);
 }
 template <typename T>
 __global__ void k_mac_prolong(lvl_dev F, lvl_dev C, T *__restrict__ x, const T *__restrict__ xc) {
@@ -176,7 +176,9 @@ static dim3 blk3() { return dim3(32, 4, 2); }
 static dim3 grid3(int a, int b, int c) { return dim3((a + 31) / 32, (b + 3) / 4, (c + 1) / 2); }
 // one plane's line of points (mg_body.cuh) per block row: every point, or one
 // colour's
-static dim3 grid_line(const mg_level &L) { return dim3((L.n[0] * L.n[1] + 255) / 256, L.n[2]); }
+static dim3 grid_line(const mg_level &L, int pz = 1) {
+    return dim3((L.n[0] * L.n[1] + 255) / 256, (L.n[2] + pz - 1) / pz);
+}
 static dim3 grid_colour(mg_kind kind, const mg_level &L) {
     const int rows = kind == MG_MAC ? L.n[1] : (L.n[1] + 1) / 2;
     return dim3(((L.n[0] + 1) / 2 * rows + 255) / 256, L.n[2]);
@@ -536,9 +538,14 @@ int mg_solver::smooth(int l, int sweeps, int cur, cudaStream_t st) {
             }
         } else {
             const dim3 g = grid_colour(kind, L);
+            const int pz = march_planes(L.npts() / 4);
+            const dim3 gm(g.x, (g.y + pz - 1) / pz);
             for (int c = 0; c < 4; c++) {
                 if (timed) prof->begin(st);
-                LAUNCH(k_fem_gs<double><<<g, 256, 0, st>>>(d, xb[cur], L.r, c, L.ri, line_inv((L.n[0] + 1) / 2)));
+                if (pz > 1)
+                    LAUNCH((k_fem_gs<double, true><<<gm, 256, 0, st>>>(d, xb[cur], L.r, c, L.ri, line_inv((L.n[0] + 1) / 2), pz)));
+                else
+                    LAUNCH((k_fem_gs<double, false><<<g, 256, 0, st>>>(d, xb[cur], L.r, c, L.ri, line_inv((L.n[0] + 1) / 2), 1)));
                 if (timed) prof->end(st, npts / 4, 8.0 * (npts + npts / 4 + npts / 4));
             }
         }
@@ -567,9 +574,14 @@ int mg_solver::smooth_f32(int l, int sweeps, int cur, cudaStream_t st) {
             }
         } else {
             const dim3 g = grid_colour(kind, L);
+            const int pz = march_planes(L.npts() / 4);
+            const dim3 gm(g.x, (g.y + pz - 1) / pz);
             for (int c = 0; c < 4; c++) {
                 if (timed) prof->begin(st);
-                LAUNCH(k_fem_gs<float><<<g, 256, 0, st>>>(d, xb[cur], L.rs, c, L.ris, line_inv((L.n[0] + 1) / 2)));
+                if (pz > 1)
+                    LAUNCH((k_fem_gs<float, true><<<gm, 256, 0, st>>>(d, xb[cur], L.rs, c, L.ris, line_inv((L.n[0] + 1) / 2), pz)));
+                else
+                    LAUNCH((k_fem_gs<float, false><<<g, 256, 0, st>>>(d, xb[cur], L.rs, c, L.ris, line_inv((L.n[0] + 1) / 2), 1)));
                 if (timed) prof->end(st, npts / 4, 4.0 * (npts + npts / 4 + npts / 4));
             }
         }
@@ -644,10 +656,14 @@ int mg_solver::cycle(int l, cudaStream_t st) {
     lvl_dev cd = dev_of(C);
     const dim3 gc = grid3(C.n[0], C.n[1], C.n[2]);
     if (kind == MG_MAC) {
-        LAUNCH((k_resid<double, 0><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]))));
+        LAUNCH((k_resid<double, 0, false><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]), 1)));
         LAUNCH(k_mac_restrict<double><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.r, C.x));
     } else {
-        LAUNCH((k_resid<double, 1><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]))));
+        const int pz = march_planes(F.npts());
+        if (pz > 1)
+            LAUNCH((k_resid<double, 1, true><<<grid_line(F, pz), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]), pz)));
+        else
+            LAUNCH((k_resid<double, 1, false><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]), 1)));
         LAUNCH(k_fem_restrict<double><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.r, C.x));
     }
     const int cc = cycle(l + 1, st);
@@ -680,10 +696,14 @@ int mg_solver::cycle_f32(int l, cudaStream_t st) {
     lvl_dev cd = dev_of(C);
     const dim3 gc = grid3(C.n[0], C.n[1], C.n[2]);
     if (kind == MG_MAC) {
-        LAUNCH((k_resid<float, 0><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]))));
+        LAUNCH((k_resid<float, 0, false><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]), 1)));
         LAUNCH(k_mac_restrict<float><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.rs, C.xs));
     } else {
-        LAUNCH((k_resid<float, 1><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]))));
+        const int pz = march_planes(F.npts());
+        if (pz > 1)
+            LAUNCH((k_resid<float, 1, true><<<grid_line(F, pz), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]), pz)));
+        else
+            LAUNCH((k_resid<float, 1, false><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]), 1)));
         LAUNCH(k_fem_restrict<float><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.rs, C.xs));
     }
     const int cc = cycle_f32(l + 1, st);
@@ -701,8 +721,10 @@ void mg_solver::refine_step(cudaStream_t st) {
     size_t n = F.npts();
     unsigned nb = (unsigned)((n + 511) / 512);
     // FP64 residual -> FP32 right-hand side, FP32 start value zero (one pass)
-    if (kind == MG_MAC) LAUNCH((k_resid_to_f32<0><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]))));
-    else LAUNCH((k_resid_to_f32<1><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]))));
+    const int pz = march_planes(n);
+    if (kind == MG_MAC) LAUNCH((k_resid_to_f32<0, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]), 1)));
+    else if (pz > 1) LAUNCH((k_resid_to_f32<1, true><<<grid_line(F, pz), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]), pz)));
+    else LAUNCH((k_resid_to_f32<1, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]), 1)));
     const int cur = cycle_f32(0, st);
     LAUNCH(k_add_f32<<<nb, 256, 0, st>>>(F.x, cur ? F.ress : F.xs, n));
 }
@@ -755,8 +777,10 @@ void mg_solver::launch_body(cudaStream_t st, bool armed, unsigned long long h) {
     iterate(st);
     mg_level &F = lv[0];
     lvl_dev fd = dev_of(F);
-    if (kind == MG_MAC) LAUNCH((k_resid_ctl<0><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]))));
-    else LAUNCH((k_resid_ctl<1><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]))));
+    const int pz = march_planes(F.npts());
+    if (kind == MG_MAC) LAUNCH((k_resid_ctl<0, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]), 1)));
+    else if (pz > 1) LAUNCH((k_resid_ctl<1, true><<<grid_line(F, pz), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]), pz)));
+    else LAUNCH((k_resid_ctl<1, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]), 1)));
     LAUNCH(k_mg_ctl<<<1, 1, 0, st>>>(ctl, d_max, max_norm_tol, rtol, exact ? 1 : 0, h, armed ? 1 : 0));
 }
 

@@ -41,26 +41,26 @@ __global__ void __launch_bounds__(256) k_mac_rb_b(lvl_dev L, T *const *x, T *con
     MGB_LINE
     body_mac_rb<T>(L, x[b_], r[b_], colour, ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
 }
-template <typename T>
+template <typename T, bool MARCH>
 __global__ void __launch_bounds__(256) k_fem_gs_b(lvl_dev L, T *const *x, T *const *r, const T *const *ri, int colour,
-                                                  const int *run, unsigned inv) {
+                                                  const int *run, unsigned inv, int pz) {
     MGB_LINE
-    body_fem_gs<T>(L, x[b_], r[b_], colour, ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
+    body_fem_gs<T, MARCH>(L, x[b_], r[b_], colour, ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y, pz);
 }
-template <typename T, int KIND>
+template <typename T, int KIND, bool MARCH>
 __global__ void __launch_bounds__(256) k_resid_b(lvl_dev L, T *const *x, T *const *r, T *const *res,
-                                                 const T *const *ri, const int *run, unsigned inv) {
+                                                 const T *const *ri, const int *run, unsigned inv, int pz) {
     MGB_LINE
-    body_resid<T, KIND>(L, x[b_], r[b_], res[b_], ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
+    body_resid<T, KIND, MARCH>(L, x[b_], r[b_], res[b_], ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y, pz);
 }
 // the control's residual: only for scenes whose control will read it
-template <int KIND>
+template <int KIND, bool MARCH>
 __global__ void __launch_bounds__(256) k_resid_ctl_b(lvl_dev L, double *const *x, double *const *r,
                                                      const double *const *ri, unsigned long long *const *mx,
-                                                     mg_ctl *const *ctl, const int *run, unsigned inv) {
+                                                     mg_ctl *const *ctl, const int *run, unsigned inv, int pz) {
     MGB_LINE
     if (!ctl[b_]->need_res) return;
-    block_max_into(body_resid_max<KIND>(L, x[b_], r[b_], ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y),
+    block_max_into(body_resid_max<KIND, MARCH>(L, x[b_], r[b_], ri ? ri[b_] : nullptr, inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y, pz),
                    mx[b_]);
 }
 template <typename T>
@@ -75,12 +75,12 @@ __global__ void k_fem_restrict_b(lvl_dev F, lvl_dev C, T *const *res, T *const *
     MGB_SCENE(zb)
     body_fem_restrict<T>(F, C, res[b_], rc[b_], xc[b_], blockIdx.x, blockIdx.y, bz_);
 }
-template <int KIND>
+template <int KIND, bool MARCH>
 __global__ void __launch_bounds__(256) k_resid_to_f32_b(lvl_dev L, double *const *x, double *const *r,
                                                         const double *const *ri, float *const *rs, float *const *xs,
-                                                        const int *run, unsigned inv) {
+                                                        const int *run, unsigned inv, int pz) {
     MGB_LINE
-    body_resid_to_f32<KIND>(L, x[b_], r[b_], ri ? ri[b_] : nullptr, rs[b_], xs[b_], inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y);
+    body_resid_to_f32<KIND, MARCH>(L, x[b_], r[b_], ri ? ri[b_] : nullptr, rs[b_], xs[b_], inv, blockIdx.x * 256 + threadIdx.x, blockIdx.y, pz);
 }
 template <typename T>
 __global__ void k_mac_prolong_b(lvl_dev F, lvl_dev C, T *const *x, T *const *xc, const int *run, int zb) {
@@ -322,9 +322,12 @@ static int smooth_b(mg_group &g, int l, int sweeps, int cur, cudaStream_t st, T 
             const bool mac = g.kind == MG_MAC;
             const int rows = mac ? L.n[1] : (L.n[1] + 1) / 2, h = (L.n[0] + 1) / 2;
             const dim3 gr((h * rows + 255) / 256, L.n[2], g.B);
+            const int pz = march_planes(L.npts() * g.B / 4);
+            const dim3 gm(gr.x, (L.n[2] + pz - 1) / pz, g.B);
             for (int c = 0; c < (mac ? 2 : 4); c++) {
                 if (mac) k_mac_rb_b<T><<<gr, 256, 0, st>>>(d, xb[cur], r, ri, c, g.run, line_inv(h));
-                else k_fem_gs_b<T><<<gr, 256, 0, st>>>(d, xb[cur], r, ri, c, g.run, line_inv(h));
+                else if (pz > 1) k_fem_gs_b<T, true><<<gm, 256, 0, st>>>(d, xb[cur], r, ri, c, g.run, line_inv(h), pz);
+                else k_fem_gs_b<T, false><<<gr, 256, 0, st>>>(d, xb[cur], r, ri, c, g.run, line_inv(h), 1);
                 g.body_kernels++;
             }
         }
@@ -368,10 +371,15 @@ static int cycle_b(mg_group &g, int l, cudaStream_t st) {
     const dim3 gr((F.n[0] * F.n[1] + 255) / 256, F.n[2], g.B),
                gf = ggrid(F.n[0], C.n[1], C.n[2], g.B, zbf), gc = ggrid(C.n[0], C.n[1], C.n[2], g.B, zbc);
     if (g.kind == MG_MAC) {
-        k_resid_b<T, 0><<<gr, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]));
+        k_resid_b<T, 0, false><<<gr, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]), 1);
         k_mac_restrict_b<T><<<gc, gblk(), 0, st>>>(ldv(F), ldv(C), xb[cur ^ 1], Rr(l + 1), X(l + 1), g.run, zbc);
     } else {
-        k_resid_b<T, 1><<<gr, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]));
+        const int pz = march_planes(F.npts() * g.B);
+        const dim3 gm(gr.x, (F.n[2] + pz - 1) / pz, g.B);
+        if (pz > 1)
+            k_resid_b<T, 1, true><<<gm, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]), pz);
+        else
+            k_resid_b<T, 1, false><<<gr, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]), 1);
         k_fem_restrict_b<T><<<gc, gblk(), 0, st>>>(ldv(F), ldv(C), xb[cur ^ 1], Rr(l + 1), X(l + 1), g.run, zbc);
     }
     g.body_kernels += 2;
@@ -400,10 +408,11 @@ void mg_group::iterate(cudaStream_t st) {
     const size_t n = F.npts();
     const dim3 g1((unsigned)((n + 511) / 512), B);
     // FP64 residual -> FP32 right-hand side, FP32 start value zero (one pass)
-    if (kind == MG_MAC)
-        k_resid_to_f32_b<0><<<gf, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]));
-    else
-        k_resid_to_f32_b<1><<<gf, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]));
+    const int pz = march_planes(F.npts() * B);
+    const dim3 gm(gf.x, (F.n[2] + pz - 1) / pz, B);
+    if (kind == MG_MAC) k_resid_to_f32_b<0, false><<<gf, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]), 1);
+    else if (pz > 1) k_resid_to_f32_b<1, true><<<gm, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]), pz);
+    else k_resid_to_f32_b<1, false><<<gf, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]), 1);
     body_kernels++;
     const int cur = cycle_b<float>(*this, 0, st);
     k_add_f32_b<<<g1, 256, 0, st>>>(tab[0].x, cur ? tab[0].ress : tab[0].xs, n, run);
@@ -425,10 +434,11 @@ int mg_group::capture(cudaStream_t cur, graph_builder &gb) {
     iterate(body);
     const mg_level &F = lv[0];
     const dim3 gf((F.n[0] * F.n[1] + 255) / 256, F.n[2], B);
-    if (kind == MG_MAC)
-        k_resid_ctl_b<0><<<gf, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]));
-    else
-        k_resid_ctl_b<1><<<gf, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]));
+    const int pz = march_planes(F.npts() * B);
+    const dim3 gm(gf.x, (F.n[2] + pz - 1) / pz, B);
+    if (kind == MG_MAC) k_resid_ctl_b<0, false><<<gf, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]), 1);
+    else if (pz > 1) k_resid_ctl_b<1, true><<<gm, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]), pz);
+    else k_resid_ctl_b<1, false><<<gf, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]), 1);
     k_mgb_ctl<<<1, 1024, 0, body>>>(ctls, mx, run, B, tol, rtol, exact ? 1 : 0, h);
     body_kernels += 2;
     gb.close(body);

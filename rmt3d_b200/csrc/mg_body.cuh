@@ -33,16 +33,141 @@ __device__ __forceinline__ void body_mac_rb(lvl_dev L, T *__restrict__ x, const 
     x[id] = (r[id] - s) / diag;
 }
 
+// A column of FEM nodes (i, j), planes k0 .. k1-1: emit(k, sum, diag, r,
+// x) for each in turn (x only with OWN).  The eight neighbour columns slide through registers, nine loads a
+// node instead of 21 (with variable density 13 instead of 29); sums and their
+// order are those of fem_offdiag and fem_offdiag_vd.  No neighbour column is of
+// the node's colour, so a pass may update the column as it goes; a plane's
+// loads are issued ahead of the sums and the store of the plane before it.
+template <typename T, bool VD, bool OWN, typename F>
+__device__ __forceinline__ void fem_march(const lvl_dev &L, const T *x, const T *__restrict__ r, const T *__restrict__ ri, int i, int j, int k0,
+                                          int k1, F emit) {
+    const int sy = L.n0, sz = L.n0 * L.n1;
+    const int xl = nb_lo(i, L.n0, L.p0, 1), xh = nb_hi(i, L.n0, L.p0, 1), yl = nb_lo(j, L.n1, L.p1, sy),
+              yh = nb_hi(j, L.n1, L.p1, sy);
+    // 0..3: (-,-) (+,-) (-,+) (+,+); 4..7: (-,0) (+,0) (0,-) (0,+)
+    const int off[8] = {yl + xl, yl + xh, yh + xl, yh + xh, xl, xh, yl, yh};
+    const T *c = x + i + sy * j + (size_t)sz * k0;
+    const int zl = nb_lo(k0, L.n2, L.p2, sz);
+    T w0[8], w1[8], w2[8], w3[8];
+    const int zf = nb_hi(k0, L.n2, L.p2, sz);
+#pragma unroll
+    for (int q = 0; q < 8; q++) w0[q] = c[zl + off[q]], w1[q] = c[off[q]], w2[q] = c[zf + off[q]];
+    T rv = r[i + sy * j + (size_t)sz * k0], xv = OWN ? c[0] : (T)0;
+    const bool inside = i > 0 && i < L.n0 - 1 && j > 0 && j < L.n1 - 1;
+    const int ncx = L.p0 ? L.n0 : L.n0 - 1, ncy = L.p1 ? L.n1 : L.n1 - 1, ncz = L.p2 ? L.n2 : L.n2 - 1;
+    T u[4], v[4];
+    int co[4];  // the column's cells of a layer, (y, x); -1: none
+    if (VD) {
+        const int i0 = i > 0 ? i - 1 : (L.p0 ? ncx - 1 : -1), i1 = i < ncx ? i : -1;
+        const int j0 = j > 0 ? j - 1 : (L.p1 ? ncy - 1 : -1), j1 = j < ncy ? j : -1;
+        co[0] = (i0 | j0) >= 0 ? i0 + ncx * j0 : -1;
+        co[1] = (i1 | j0) >= 0 ? i1 + ncx * j0 : -1;
+        co[2] = (i0 | j1) >= 0 ? i0 + ncx * j1 : -1;
+        co[3] = (i1 | j1) >= 0 ? i1 + ncx * j1 : -1;
+        const int kc = k0 > 0 ? k0 - 1 : (L.p2 ? ncz - 1 : -1);
+#pragma unroll
+        for (int q = 0; q < 4; q++) u[q] = (co[q] | kc) >= 0 ? ri[co[q] + (size_t)ncx * ncy * kc] : (T)0;
+    }
+    for (int k = k0; k < k1; k++, c += sz) {
+        T rn = 0, xn = 0;
+        if (k + 1 < k1) {
+            const int zh = sz + nb_hi(k + 1, L.n2, L.p2, sz);
+#pragma unroll
+            for (int q = 0; q < 8; q++) w3[q] = c[zh + off[q]];
+            rn = r[i + sy * j + (size_t)sz * (k + 1)];
+            if (OWN) xn = c[sz];
+        }
+        T s, diag;
+        if (VD) {
+            const int kc = k < ncz ? k : -1;
+#pragma unroll
+            for (int q = 0; q < 4; q++) v[q] = (co[q] | kc) >= 0 ? ri[co[q] + (size_t)ncx * ncy * kc] : (T)0;
+            s = 0;
+            s += -u[0] * w0[0];
+            s += -(u[0] + u[1]) * w0[6];
+            s += -u[1] * w0[1];
+            s += -(u[0] + u[2]) * w0[4];
+            s += -(u[1] + u[3]) * w0[5];
+            s += -u[2] * w0[2];
+            s += -(u[2] + u[3]) * w0[7];
+            s += -u[3] * w0[3];
+            s += -(u[0] + v[0]) * w1[0];
+            s += -(u[1] + v[1]) * w1[1];
+            s += -(u[2] + v[2]) * w1[2];
+            s += -(u[3] + v[3]) * w1[3];
+            s += -v[0] * w2[0];
+            s += -(v[0] + v[1]) * w2[6];
+            s += -v[1] * w2[1];
+            s += -(v[0] + v[2]) * w2[4];
+            s += -(v[1] + v[3]) * w2[5];
+            s += -v[2] * w2[2];
+            s += -(v[2] + v[3]) * w2[7];
+            s += -v[3] * w2[3];
+            T c8 = 0;
+#pragma unroll
+            for (int q = 0; q < 4; q++) c8 += u[q];
+#pragma unroll
+            for (int q = 0; q < 4; q++) c8 += v[q];
+            diag = (T)4 * c8;
+#pragma unroll
+            for (int q = 0; q < 4; q++) u[q] = v[q];
+        } else if (inside && k > 0 && k < L.n2 - 1) {
+            T e = (w1[0] + w1[1]) + (w1[2] + w1[3]);
+            e += (w0[4] + w0[5]) + (w0[6] + w0[7]);
+            e += (w2[4] + w2[5]) + (w2[6] + w2[7]);
+            T q = (w0[0] + w0[1]) + (w0[2] + w0[3]);
+            q += (w2[0] + w2[1]) + (w2[2] + w2[3]);
+            s = (T)-2 * e - q;
+            diag = (T)32;
+        } else {
+            s = fem_rim_sum(L, i, j, k, w0[0], w0[6], w0[1], w0[4], w0[5], w0[2], w0[7], w0[3], w1[0], w1[1], w1[2],
+                            w1[3], w2[0], w2[6], w2[1], w2[4], w2[5], w2[2], w2[7], w2[3], diag);
+        }
+        emit(k, s, diag, rv, xv);
+#pragma unroll
+        for (int q = 0; q < 8; q++) w0[q] = w1[q], w1[q] = w2[q], w2[q] = w3[q];
+        rv = rn, xv = xn;
+    }
+}
+
+// Planes per thread of a FEM phase over `points` points; 1: point by point.  A
+// point by itself waits on its 21 loads and little else; marching reads less
+// and keeps a plane of loads in flight, but leaves fewer threads.  The line lies
+// at 200,000 threads and 16 planes (B200, 193^3 nodes): FP64 residual to FP32
+// 126 -> 79 us (8 planes 84, 4 planes 93), its max norm 151 -> 77 us, FP32
+// residual of 193^3 and 97^3 38 -> 27 us, FP32 colour pass of 193^3 19 -> 14 us.
+// Below it the two are level: FP32 colour pass of 97^3 variable density 5.2 us
+// either way, with a quarter of the threads 5.8 us.
+inline int march_planes(size_t points) {
+    const size_t p = points / 200000;
+    return p < 2 ? 1 : p > 16 ? 16 : (int)p;
+}
+
 // The Q1 stencil couples a node only to its edge and corner neighbours (the
 // face entries are zero), so colouring by the parities of i and j alone never
 // puts two coupled nodes in one colour: four colour passes are an exact
 // Gauss-Seidel sweep.  The line of a colour has (n0 + 1) / 2 nodes a row for
 // either parity of i.
-template <typename T>
-__device__ __forceinline__ void body_fem_gs(lvl_dev L, T *__restrict__ x, const T *__restrict__ r, int colour, const T *__restrict__ ri, unsigned inv, int pt, int k) {
+template <typename T, bool MARCH>
+__device__ __forceinline__ void body_fem_gs(lvl_dev L, T *x, const T *__restrict__ r, int colour, const T *__restrict__ ri, unsigned inv, int pt, int kb, int pz) {
     const int h = (L.n0 + 1) >> 1, b = line_row(pt, inv);
     const int i = 2 * (pt - b * h) + (colour & 1), j = 2 * b + (colour >> 1);
     if (i >= L.n0 || j >= L.n1) return;
+    if (MARCH) {
+        const int k0 = kb * pz, k1 = min(k0 + pz, L.n2), h = fem_walls(L, i, j);
+        const int id0 = i + L.n0 * j, sz = L.n0 * L.n1;
+        if (ri)
+            fem_march<T, true, false>(L, x, r, ri, i, j, k0, k1,
+                                      [&](int k, T s, T diag, T rv, T) { x[id0 + sz * k] = (rv - s) / diag; });
+        else
+            fem_march<T, false, false>(L, x, r, ri, i, j, k0, k1, [&](int k, T s, T, T rv, T) {
+                const int w = h + (!L.p2 && (k == 0 || k == L.n2 - 1) ? 1 : 0);
+                x[id0 + sz * k] = (rv - s) * ((T)(1 << w) * (T)0.03125);
+            });
+        return;
+    }
+    const int k = kb;
     T diag;
     const int id = i + L.n0 * (j + L.n1 * k);
     if (ri) {
@@ -55,11 +180,19 @@ __device__ __forceinline__ void body_fem_gs(lvl_dev L, T *__restrict__ x, const 
 }
 
 // ---- residuals: r - A x into emit(index, value) ------------------------------
-template <typename T, int KIND, typename F>
+template <typename T, int KIND, bool MARCH, typename F>
 __device__ __forceinline__ void body_resid_emit(const lvl_dev &L, const T *__restrict__ x, const T *__restrict__ r,
-                                                const T *__restrict__ ri, unsigned inv, int pt, int k, F emit) {
+                                                const T *__restrict__ ri, unsigned inv, int pt, int kb, int pz, F emit) {
     const int j = line_row(pt, inv), i = pt - j * L.n0;
     if (j >= L.n1) return;
+    if (MARCH && KIND == 1) {
+        const int k0 = kb * pz, k1 = min(k0 + pz, L.n2), id0 = i + L.n0 * j, sz = L.n0 * L.n1;
+        auto f = [&](int k, T s, T diag, T rv, T xv) { emit(id0 + sz * k, rv - s - diag * xv); };
+        if (ri) fem_march<T, true, true>(L, x, r, ri, i, j, k0, k1, f);
+        else fem_march<T, false, true>(L, x, r, ri, i, j, k0, k1, f);
+        return;
+    }
+    const int k = kb;
     T diag;
     const T s = op_offdiag<T>(KIND, L, x, ri, i, j, k, diag);
     const int id = i + L.n0 * (j + L.n1 * k);
@@ -67,21 +200,21 @@ __device__ __forceinline__ void body_resid_emit(const lvl_dev &L, const T *__res
 }
 
 // res = r - A x
-template <typename T, int KIND>
+template <typename T, int KIND, bool MARCH>
 __device__ __forceinline__ void body_resid(lvl_dev L, const T *__restrict__ x, const T *__restrict__ r,
-                                           T *__restrict__ res, const T *__restrict__ ri, unsigned inv, int pt, int k) {
-    body_resid_emit<T, KIND>(L, x, r, ri, inv, pt, k, [&](int id, T v) { res[id] = v; });
+                                           T *__restrict__ res, const T *__restrict__ ri, unsigned inv, int pt, int k, int pz) {
+    body_resid_emit<T, KIND, MARCH>(L, x, r, ri, inv, pt, k, pz, [&](int id, T v) { res[id] = v; });
 }
 
 // max |r - A x| over the calling thread's points, as the ordered bit pattern
 // (NaN the largest)
-template <int KIND>
+template <int KIND, bool MARCH>
 __device__ __forceinline__ unsigned long long body_resid_max(lvl_dev L, const double *__restrict__ x,
                                                              const double *__restrict__ r,
                                                              const double *__restrict__ ri, unsigned inv, int pt,
-                                                             int k) {
+                                                             int k, int pz) {
     unsigned long long m = 0;
-    body_resid_emit<double, KIND>(L, x, r, ri, inv, pt, k, [&](int, double v) {
+    body_resid_emit<double, KIND, MARCH>(L, x, r, ri, inv, pt, k, pz, [&](int, double v) {
         const double a = fabs(v);
         const unsigned long long b = a != a ? 0x7ff8000000000000ULL : (unsigned long long)__double_as_longlong(a);
         m = b > m ? b : m;
@@ -92,12 +225,12 @@ __device__ __forceinline__ unsigned long long body_resid_max(lvl_dev L, const do
 // The mixed form's FP64 residual handed to the FP32 cycle in one pass: the
 // residual r - A x in FP64, rounded to FP32 as the cycle's right-hand side,
 // and the cycle's FP32 start value zeroed.
-template <int KIND>
+template <int KIND, bool MARCH>
 __device__ __forceinline__ void body_resid_to_f32(lvl_dev L, const double *__restrict__ x,
                                                   const double *__restrict__ r, const double *__restrict__ ri,
                                                   float *__restrict__ rs, float *__restrict__ xs, unsigned inv,
-                                                  int pt, int k) {
-    body_resid_emit<double, KIND>(L, x, r, ri, inv, pt, k, [&](int id, double v) {
+                                                  int pt, int k, int pz) {
+    body_resid_emit<double, KIND, MARCH>(L, x, r, ri, inv, pt, k, pz, [&](int id, double v) {
         rs[id] = (float)v;
         xs[id] = 0;
     });

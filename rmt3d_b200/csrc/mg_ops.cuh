@@ -65,28 +65,12 @@ __device__ __forceinline__ T mac_offdiag(const lvl_dev L, const T *__restrict__ 
     return s;
 }
 
+// the constant-density FEM sum of a node on the rim of the level, term by
+// term: a.., b.., d.. the planes below, of and above the node, digits x and y
 template <typename T>
-__device__ __forceinline__ T fem_offdiag(const lvl_dev L, const T *__restrict__ x, int i, int j, int k, T &diag) {
-    // edges -2, corners -1, faces 0
-    const int sy = L.n0, sz = L.n0 * L.n1;
-    const int xl = nb_lo(i, L.n0, L.p0, 1), xh = nb_hi(i, L.n0, L.p0, 1);
-    const T *c = x + i + sy * j + sz * k;
-    const T *y0 = c + nb_lo(j, L.n1, L.p1, sy), *y2 = c + nb_hi(j, L.n1, L.p1, sy);
-    const int zl = nb_lo(k, L.n2, L.p2, sz), zh = nb_hi(k, L.n2, L.p2, sz);
-    const T a00 = y0[zl + xl], a10 = y0[zl], a20 = y0[zl + xh], a01 = c[zl + xl], a21 = c[zl + xh], a02 = y2[zl + xl],
-            a12 = y2[zl], a22 = y2[zl + xh];
-    const T b00 = y0[xl], b20 = y0[xh], b02 = y2[xl], b22 = y2[xh];
-    const T d00 = y0[zh + xl], d10 = y0[zh], d20 = y0[zh + xh], d01 = c[zh + xl], d21 = c[zh + xh], d02 = y2[zh + xl],
-            d12 = y2[zh], d22 = y2[zh + xh];
-    if (i > 0 && i < L.n0 - 1 && j > 0 && j < L.n1 - 1 && k > 0 && k < L.n2 - 1) {
-        T e = (b00 + b20) + (b02 + b22);
-        e += (a01 + a21) + (a10 + a12);
-        e += (d01 + d21) + (d10 + d12);
-        T q = (a00 + a20) + (a02 + a22);
-        q += (d00 + d20) + (d02 + d22);
-        diag = (T)32;
-        return (T)-2 * e - q;
-    }
+__device__ __forceinline__ T fem_rim_sum(const lvl_dev &L, int i, int j, int k, T a00, T a10, T a20, T a01, T a21, T a02,
+                                         T a12, T a22, T b00, T b20, T b02, T b22, T d00, T d10, T d20, T d01, T d21,
+                                         T d02, T d12, T d22, T &diag) {
     // 1 where the neighbour on that side exists; an entry is halved once per
     // wall plane the node lies on along an axis it does not move along
     const bool wx = !L.p0 && (i == 0 || i == L.n0 - 1), wy = !L.p1 && (j == 0 || j == L.n1 - 1),
@@ -119,6 +103,37 @@ __device__ __forceinline__ T fem_offdiag(const lvl_dev L, const T *__restrict__ 
     s += -(p22 * z1) * d22;
     diag = (T)(32 >> ((int)wx + (int)wy + (int)wz));
     return s;
+}
+
+template <typename T>
+__device__ __forceinline__ T fem_offdiag(const lvl_dev L, const T *__restrict__ x, int i, int j, int k, T &diag) {
+    // edges -2, corners -1, faces 0
+    const int sy = L.n0, sz = L.n0 * L.n1;
+    const int xl = nb_lo(i, L.n0, L.p0, 1), xh = nb_hi(i, L.n0, L.p0, 1);
+    const T *c = x + i + sy * j + sz * k;
+    const T *y0 = c + nb_lo(j, L.n1, L.p1, sy), *y2 = c + nb_hi(j, L.n1, L.p1, sy);
+    const int zl = nb_lo(k, L.n2, L.p2, sz), zh = nb_hi(k, L.n2, L.p2, sz);
+    const T a00 = y0[zl + xl], a10 = y0[zl], a20 = y0[zl + xh], a01 = c[zl + xl], a21 = c[zl + xh], a02 = y2[zl + xl],
+            a12 = y2[zl], a22 = y2[zl + xh];
+    const T b00 = y0[xl], b20 = y0[xh], b02 = y2[xl], b22 = y2[xh];
+    const T d00 = y0[zh + xl], d10 = y0[zh], d20 = y0[zh + xh], d01 = c[zh + xl], d21 = c[zh + xh], d02 = y2[zh + xl],
+            d12 = y2[zh], d22 = y2[zh + xh];
+    if (i > 0 && i < L.n0 - 1 && j > 0 && j < L.n1 - 1 && k > 0 && k < L.n2 - 1) {
+        T e = (b00 + b20) + (b02 + b22);
+        e += (a01 + a21) + (a10 + a12);
+        e += (d01 + d21) + (d10 + d12);
+        T q = (a00 + a20) + (a02 + a22);
+        q += (d00 + d20) + (d02 + d22);
+        diag = (T)32;
+        return (T)-2 * e - q;
+    }
+    return fem_rim_sum(L, i, j, k, a00, a10, a20, a01, a21, a02, a12, a22, b00, b20, b02, b22, d00, d10, d20, d01, d21,
+                       d02, d12, d22, diag);
+}
+
+// walled axes x and y on whose end planes a FEM node lies
+__device__ __forceinline__ int fem_walls(const lvl_dev &L, int i, int j) {
+    return (!L.p0 && (i == 0 || i == L.n0 - 1)) + (!L.p1 && (j == 0 || j == L.n1 - 1));
 }
 
 // 1 / diag of the constant-density FEM stencil at node (i, j, k).  diag is
