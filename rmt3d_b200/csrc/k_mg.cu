@@ -656,7 +656,11 @@ int mg_solver::cycle(int l, cudaStream_t st) {
     lvl_dev cd = dev_of(C);
     const dim3 gc = grid3(C.n[0], C.n[1], C.n[2]);
     if (kind == MG_MAC) {
-        LAUNCH((k_resid<double, 0, false><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]), 1)));
+        const int pz = F.ri ? 1 : march_planes(F.npts());
+        if (pz > 1)
+            LAUNCH((k_resid<double, 0, true><<<grid_line(F, pz), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]), pz)));
+        else
+            LAUNCH((k_resid<double, 0, false><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.r, xb[cur ^ 1], F.ri, line_inv(F.n[0]), 1)));
         LAUNCH(k_mac_restrict<double><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.r, C.x));
     } else {
         const int pz = march_planes(F.npts());
@@ -696,7 +700,11 @@ int mg_solver::cycle_f32(int l, cudaStream_t st) {
     lvl_dev cd = dev_of(C);
     const dim3 gc = grid3(C.n[0], C.n[1], C.n[2]);
     if (kind == MG_MAC) {
-        LAUNCH((k_resid<float, 0, false><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]), 1)));
+        const int pz = F.ris ? 1 : march_planes(F.npts());
+        if (pz > 1)
+            LAUNCH((k_resid<float, 0, true><<<grid_line(F, pz), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]), pz)));
+        else
+            LAUNCH((k_resid<float, 0, false><<<grid_line(F), 256, 0, st>>>(fd, xb[cur], F.rs, xb[cur ^ 1], F.ris, line_inv(F.n[0]), 1)));
         LAUNCH(k_mac_restrict<float><<<gc, blk3(), 0, st>>>(fd, cd, xb[cur ^ 1], C.rs, C.xs));
     } else {
         const int pz = march_planes(F.npts());
@@ -721,8 +729,9 @@ void mg_solver::refine_step(cudaStream_t st) {
     size_t n = F.npts();
     unsigned nb = (unsigned)((n + 511) / 512);
     // FP64 residual -> FP32 right-hand side, FP32 start value zero (one pass)
-    const int pz = march_planes(n);
-    if (kind == MG_MAC) LAUNCH((k_resid_to_f32<0, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]), 1)));
+    const int pz = kind == MG_MAC && F.ri ? 1 : march_planes(n);
+    if (kind == MG_MAC && pz > 1) LAUNCH((k_resid_to_f32<0, true><<<grid_line(F, pz), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]), pz)));
+    else if (kind == MG_MAC) LAUNCH((k_resid_to_f32<0, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]), 1)));
     else if (pz > 1) LAUNCH((k_resid_to_f32<1, true><<<grid_line(F, pz), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]), pz)));
     else LAUNCH((k_resid_to_f32<1, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, F.ri, F.rs, F.xs, line_inv(F.n[0]), 1)));
     const int cur = cycle_f32(0, st);
@@ -777,8 +786,9 @@ void mg_solver::launch_body(cudaStream_t st, bool armed, unsigned long long h) {
     iterate(st);
     mg_level &F = lv[0];
     lvl_dev fd = dev_of(F);
-    const int pz = march_planes(F.npts());
-    if (kind == MG_MAC) LAUNCH((k_resid_ctl<0, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]), 1)));
+    const int pz = kind == MG_MAC && F.ri ? 1 : march_planes(F.npts());
+    if (kind == MG_MAC && pz > 1) LAUNCH((k_resid_ctl<0, true><<<grid_line(F, pz), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]), pz)));
+    else if (kind == MG_MAC) LAUNCH((k_resid_ctl<0, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]), 1)));
     else if (pz > 1) LAUNCH((k_resid_ctl<1, true><<<grid_line(F, pz), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]), pz)));
     else LAUNCH((k_resid_ctl<1, false><<<grid_line(F), 256, 0, st>>>(fd, F.x, F.r, d_max, F.ri, ctl, line_inv(F.n[0]), 1)));
     LAUNCH(k_mg_ctl<<<1, 1, 0, st>>>(ctl, d_max, max_norm_tol, rtol, exact ? 1 : 0, h, armed ? 1 : 0));

@@ -370,12 +370,15 @@ static int cycle_b(mg_group &g, int l, cudaStream_t st) {
     int zbf, zbc;
     const dim3 gr((F.n[0] * F.n[1] + 255) / 256, F.n[2], g.B),
                gf = ggrid(F.n[0], C.n[1], C.n[2], g.B, zbf), gc = ggrid(C.n[0], C.n[1], C.n[2], g.B, zbc);
+    const int pz = g.kind == MG_MAC && RI(l) ? 1 : march_planes(F.npts() * g.B);
+    const dim3 gm(gr.x, (F.n[2] + pz - 1) / pz, g.B);
     if (g.kind == MG_MAC) {
-        k_resid_b<T, 0, false><<<gr, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]), 1);
+        if (pz > 1)
+            k_resid_b<T, 0, true><<<gm, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]), pz);
+        else
+            k_resid_b<T, 0, false><<<gr, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]), 1);
         k_mac_restrict_b<T><<<gc, gblk(), 0, st>>>(ldv(F), ldv(C), xb[cur ^ 1], Rr(l + 1), X(l + 1), g.run, zbc);
     } else {
-        const int pz = march_planes(F.npts() * g.B);
-        const dim3 gm(gr.x, (F.n[2] + pz - 1) / pz, g.B);
         if (pz > 1)
             k_resid_b<T, 1, true><<<gm, 256, 0, st>>>(ldv(F), xb[cur], Rr(l), xb[cur ^ 1], RI(l), g.run, line_inv(F.n[0]), pz);
         else
@@ -408,9 +411,10 @@ void mg_group::iterate(cudaStream_t st) {
     const size_t n = F.npts();
     const dim3 g1((unsigned)((n + 511) / 512), B);
     // FP64 residual -> FP32 right-hand side, FP32 start value zero (one pass)
-    const int pz = march_planes(F.npts() * B);
+    const int pz = kind == MG_MAC && tab[0].ri ? 1 : march_planes(F.npts() * B);
     const dim3 gm(gf.x, (F.n[2] + pz - 1) / pz, B);
-    if (kind == MG_MAC) k_resid_to_f32_b<0, false><<<gf, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]), 1);
+    if (kind == MG_MAC && pz > 1) k_resid_to_f32_b<0, true><<<gm, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]), pz);
+    else if (kind == MG_MAC) k_resid_to_f32_b<0, false><<<gf, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]), 1);
     else if (pz > 1) k_resid_to_f32_b<1, true><<<gm, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]), pz);
     else k_resid_to_f32_b<1, false><<<gf, 256, 0, st>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, tab[0].rs, tab[0].xs, run, line_inv(F.n[0]), 1);
     body_kernels++;
@@ -434,9 +438,10 @@ int mg_group::capture(cudaStream_t cur, graph_builder &gb) {
     iterate(body);
     const mg_level &F = lv[0];
     const dim3 gf((F.n[0] * F.n[1] + 255) / 256, F.n[2], B);
-    const int pz = march_planes(F.npts() * B);
+    const int pz = kind == MG_MAC && tab[0].ri ? 1 : march_planes(F.npts() * B);
     const dim3 gm(gf.x, (F.n[2] + pz - 1) / pz, B);
-    if (kind == MG_MAC) k_resid_ctl_b<0, false><<<gf, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]), 1);
+    if (kind == MG_MAC && pz > 1) k_resid_ctl_b<0, true><<<gm, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]), pz);
+    else if (kind == MG_MAC) k_resid_ctl_b<0, false><<<gf, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]), 1);
     else if (pz > 1) k_resid_ctl_b<1, true><<<gm, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]), pz);
     else k_resid_ctl_b<1, false><<<gf, 256, 0, body>>>(ldv(F), tab[0].x, tab[0].r, tab[0].ri, mx, ctls, run, line_inv(F.n[0]), 1);
     k_mgb_ctl<<<1, 1024, 0, body>>>(ctls, mx, run, B, tol, rtol, exact ? 1 : 0, h);

@@ -42,12 +42,7 @@ __device__ __forceinline__ int nb_lo(int c, int n, int prd, int st) { return c >
 __device__ __forceinline__ int nb_hi(int c, int n, int prd, int st) { return c < n - 1 ? st : (prd ? (1 - n) * st : -st); }
 
 template <typename T>
-__device__ __forceinline__ T mac_offdiag(const lvl_dev L, const T *__restrict__ x, int i, int j, int k, T &diag) {
-    const int sy = L.n0, sz = L.n0 * L.n1;
-    const T *c = x + i + sy * j + sz * k;
-    T xm = c[nb_lo(i, L.n0, L.p0, 1)], xp = c[nb_hi(i, L.n0, L.p0, 1)];
-    T ym = c[nb_lo(j, L.n1, L.p1, sy)], yp = c[nb_hi(j, L.n1, L.p1, sy)];
-    T zm = c[nb_lo(k, L.n2, L.p2, sz)], zp = c[nb_hi(k, L.n2, L.p2, sz)];
+__device__ __forceinline__ T mac_sum(const lvl_dev &L, int i, int j, int k, T xm, T xp, T ym, T yp, T zm, T zp, T &diag) {
     if (i > 0 && i < L.n0 - 1 && j > 0 && j < L.n1 - 1 && k > 0 && k < L.n2 - 1) {
         diag = (T)-6;
         return ((xm + xp) + (ym + yp)) + (zm + zp);
@@ -63,6 +58,16 @@ __device__ __forceinline__ T mac_offdiag(const lvl_dev L, const T *__restrict__ 
     s += c1 ? (T)0 : zp;
     diag = (T)(-6 + (int)a0 + (int)a1 + (int)b0 + (int)b1 + (int)c0 + (int)c1);
     return s;
+}
+
+template <typename T>
+__device__ __forceinline__ T mac_offdiag(const lvl_dev L, const T *__restrict__ x, int i, int j, int k, T &diag) {
+    const int sy = L.n0, sz = L.n0 * L.n1;
+    const T *c = x + i + sy * j + sz * k;
+    T xm = c[nb_lo(i, L.n0, L.p0, 1)], xp = c[nb_hi(i, L.n0, L.p0, 1)];
+    T ym = c[nb_lo(j, L.n1, L.p1, sy)], yp = c[nb_hi(j, L.n1, L.p1, sy)];
+    T zm = c[nb_lo(k, L.n2, L.p2, sz)], zp = c[nb_hi(k, L.n2, L.p2, sz)];
+    return mac_sum(L, i, j, k, xm, xp, ym, yp, zm, zp, diag);
 }
 
 // the constant-density FEM sum of a node on the rim of the level, term by

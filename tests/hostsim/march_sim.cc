@@ -1,5 +1,5 @@
-// FEM colour passes and residuals that march along z (fem_march, mg_body.cuh)
-// against the same phases point by point: the same bits for every mix of
+// FEM colour passes and residuals, and MAC residuals, that march along z
+// (fem_march and mac_march, mg_body.cuh) against the same phases point by point: the same bits for every mix of
 // periodic and walled axes, both densities, both types and every number of
 // planes a thread, the last block short.  Built with the address sanitizer,
 // each array a heap block of its own size.
@@ -83,6 +83,21 @@ static int check(const int *n, int axes, bool vd) {
     run(n[0] * n[1], n[2], 1, [&](int pt, int kb) {
         body_resid<T, 1, false>(L, x.data(), r.data(), res.data(), q, line_inv(n[0]), pt, kb, 1);
     });
+    // constant-density MAC residual (any box of at least two cells an axis)
+    std::vector<T> mres(N);
+    run(n[0] * n[1], n[2], 1, [&](int pt, int kb) {
+        body_resid<T, 0, false>(L, x.data(), r.data(), mres.data(), nullptr, line_inv(n[0]), pt, kb, 1);
+    });
+    for (int pz = 1; pz <= 16; pz++) {
+        std::vector<T> gm(N);
+        run(n[0] * n[1], n[2], pz, [&](int pt, int kb) {
+            body_resid<T, 0, true>(L, x.data(), r.data(), gm.data(), nullptr, line_inv(n[0]), pt, kb, pz);
+        });
+        if (!same(gm, mres)) {
+            printf("%d %d %d axes %d planes %d: MAC residual\n", n[0], n[1], n[2], axes, pz);
+            return 1;
+        }
+    }
     for (int pz = 1; pz <= 16; pz++) {
         std::vector<T> got(x), gres(N);
         for (int c = 0; c < 4; c++)
