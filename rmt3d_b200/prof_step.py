@@ -26,7 +26,8 @@ cfg = scenes.write(os.path.join(wd, 'w.cfg'), text)
 d = R.desc_from_cfg(cfg); d.precision = prec; d.var_den = vd
 sc = R.Scene(d)
 sc.set_schedule(vdn, vup, 0)
-sc.set_smoother(smoother)
+if smoother >= 0:  # -1: as a new scene, with the shared-memory V-cycle
+    sc.set_smoother(smoother)
 sc.prepare()
 sc.step_forward(0)
 sc.sync()
