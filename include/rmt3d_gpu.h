@@ -363,7 +363,9 @@ int rmt3d_div_u_noalloc(const int sys_size[3], const int periodic[3], const doub
  * whose PGMG smoothing is a library internal): mode 0 issues one launch per
  * colour pass of the Gauss-Seidel sweeps; mode 1 one launch per whole sweep,
  * each block staging a box with an overlapped halo in shared memory and
- * running every colour pass there.  Both give the same bits. */
+ * running every colour pass there.  Both give the same bits.  The smoother
+ * named runs on every level: a new scene's cluster launch of the levels that
+ * fit goes with either mode (rmt3d_scene_set_coarse_cluster asks for it). */
 int rmt3d_scene_set_smoother(rmt3d_scene *s, int mode);
 
 /* The part of every V-cycle on the levels of at most `pts` points, down to the
@@ -372,9 +374,11 @@ int rmt3d_scene_set_smoother(rmt3d_scene *s, int mode);
  * those levels in shared memory, instead of one full-GPU launch per phase
  * (the same bits).  Levels too large for the cluster's shared memory keep
  * per-phase launches; 0 keeps them for every level.  A new scene hands over
- * as many levels as fit, until this call, rmt3d_scene_set_smoother or a
- * one-block coarse sub-cycle (rmt3d_scene_set_schedule) chooses otherwise.
- * No counterpart in the reference. */
+ * as many levels as fit, until this call, rmt3d_scene_set_smoother (either
+ * mode) or a one-block coarse sub-cycle (rmt3d_scene_set_schedule) chooses
+ * otherwise; RMT3D_COARSE_CLUSTER_ALL, a limit no level exceeds, hands over as
+ * many again.  No counterpart in the reference. */
+#define RMT3D_COARSE_CLUSTER_ALL 2147483647
 int rmt3d_scene_set_coarse_cluster(rmt3d_scene *s, int pts);
 
 /* Block shape of the bulk stencil kernels of the step (stress, edge states,
@@ -416,7 +420,8 @@ int rmt3d_batch_scene(rmt3d_batch *b, int i, rmt3d_scene **out);
  * smoothing counts (v_down, v_up), as the reference's mg_opt searches them
  * (Utilities/mg_probs.hh:80-208), the cluster or per-phase launch of the
  * solves, the smoother (colour passes or tiled sweeps) and the coarse
- * levels run as one cluster launch per V-cycle (rmt3d_scene_set_coarse_cluster);
+ * levels run as one cluster launch per V-cycle (rmt3d_scene_set_coarse_cluster;
+ * a new scene's choice among them, and kept where no candidate runs);
  * then, under the chosen schedule, the block shape of the bulk stencil
  * kernels (rmt3d_scene_set_block_shape).  tuned_out gets 7 ints per kind:
  * (cells, v_down, v_up, cluster, smoother, coarse cluster points, block

@@ -18,7 +18,7 @@ import os
 import numpy as np
 
 from . import _lib
-from ._lib import FP64, MIXED, MIXED_BULK32, PROJECTION_ERR, REFMAP_UPDATE_ERR, STEADY_SOLN_EXIT  # noqa: F401
+from ._lib import COARSE_CLUSTER_ALL, FP64, MIXED, MIXED_BULK32, PROJECTION_ERR, REFMAP_UPDATE_ERR, STEADY_SOLN_EXIT  # noqa: F401
 from ._lib import OK as NORMAL_EXIT
 from ._lib import RMT3DError, SceneDesc
 
@@ -266,12 +266,15 @@ class Scene:
 
     def set_smoother(self, mode):
         """Multigrid smoothing: 0 one launch per colour pass, 1 one launch per
-        whole sweep on shared-memory tiles (the same bits)."""
+        whole sweep on shared-memory tiles (the same bits).  Either runs on
+        every level, until set_coarse_cluster asks for its launch again."""
         _lib.check(lib().rmt3d_scene_set_smoother(self._h, int(mode)))
 
     def set_coarse_cluster(self, pts):
-        """Run the V-cycles' levels of at most `pts` points (below the finest)
-        as one thread-block-cluster launch per cycle; 0: per-phase launches."""
+        """Run the V-cycles' levels of at most `pts` points that fit a
+        thread-block cluster's shared memory as one launch per cycle; 0:
+        per-phase launches; COARSE_CLUSTER_ALL: every level that fits, as a
+        new scene does (the same bits)."""
         _lib.check(lib().rmt3d_scene_set_coarse_cluster(self._h, int(pts)))
 
     def set_block_shape(self, shape):

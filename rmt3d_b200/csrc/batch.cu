@@ -258,12 +258,13 @@ extern "C" int rmt3d_batch_scene(rmt3d_batch *b, int i, rmt3d_scene **out) {
 // the smoothing counts (v_down, v_up), each solve as one thread-block-cluster
 // launch or as per-phase launches, and for the latter the smoother (one
 // launch per colour pass, or one per whole sweep on shared-memory tiles) and
-// the levels (none, up to 5000 or up to 40000 points) whose part of each
-// V-cycle runs as one cluster launch.  With the fastest of those, the block
-// shapes of the bulk stencil kernels are timed the same way
-// (rmt3d_scene_set_block_shape).  tuned_out (optional, 7 ints per kind:
-// cells, v_down, v_up, cluster launch, smoother, coarse cluster points,
-// block shape) receives the choices.
+// the levels (none, up to 5000 or 40000 points, or every one that fits, as a
+// new scene has it) whose part of each V-cycle runs as one cluster launch.
+// Where every candidate fails on the probe, a new scene's schedule stays.
+// With the fastest of those, the block shapes of the bulk stencil kernels are
+// timed the same way (rmt3d_scene_set_block_shape).  tuned_out (optional, 7
+// ints per kind: cells, v_down, v_up, cluster launch, smoother, coarse cluster
+// points, block shape) receives the choices.
 extern "C" int rmt3d_batch_autotune(rmt3d_batch *b, int probe_steps, int *tuned_out, int max_out, int *n_out) {
     if (!b) return rmt3d::fail(RMT3D_ERR_INVALID, "null batch");
     if (probe_steps < 1) return rmt3d::fail(RMT3D_ERR_INVALID, "probe_steps < 1");
@@ -271,7 +272,8 @@ extern "C" int rmt3d_batch_autotune(rmt3d_batch *b, int probe_steps, int *tuned_
     static const int smooth[][2] = {{2, 2}, {1, 1}, {1, 2}, {2, 1}, {3, 3}};
     // (whole solve as one cluster launch, smoother: 0 colour passes, 1 tiled
     // sweeps, largest level of the part run as one cluster launch)
-    static const int launch[][3] = {{1, 0, 0}, {0, 0, 40000}, {0, 0, 5000}, {0, 0, 0}, {0, 1, 0}};
+    static const int launch[][3] = {{1, 0, 0}, {0, 0, 40000}, {0, 0, 5000}, {0, 0, RMT3D_COARSE_CLUSTER_ALL},
+                                    {0, 0, 0}, {0, 1, 0}};
     std::map<std::array<int, 8>, int> first;
     for (size_t i = 0; i < b->descs.size(); i++)
         if (!first.count(tune_key(b->descs[i]))) first[tune_key(b->descs[i])] = (int)i;
@@ -335,10 +337,21 @@ extern "C" int rmt3d_batch_autotune(rmt3d_batch *b, int probe_steps, int *tuned_
             return bi;
         };
         std::vector<cand> cs;
-        for (auto &ln : launch)
+        // the levels a limit hands over (none: -1) and the first limit that does:
+        // another one is that candidate again
+        std::map<std::array<int, 2>, int> limit = {{{-1, -1}, 0}};
+        int all = 0;  // a new scene's
+        for (auto &ln : launch) {
+            if (ln[2] > 0) {
+                if (rmt3d_scene_set_coarse_cluster(probe, ln[2])) continue;  // clusters unavailable on this device
+                const auto at = limit.insert({rmt3d::scene_cluster_levels(probe), ln[2]});
+                if (ln[2] == RMT3D_COARSE_CLUSTER_ALL) all = at.first->second;
+                if (!at.second) continue;
+            }
             for (auto &c : smooth) cs.push_back({c[0], c[1], ln[0], ln[1], ln[2], 0, 0.0, true});
+        }
         int bi = race(cs);
-        int bd = 2, bu = 2, bc = 0, bs = 0, bcc = 0, bb = 0;
+        int bd = 2, bu = 2, bc = 0, bs = 0, bcc = all, bb = 0;
         if (bi >= 0) {
             bd = cs[bi].vd, bu = cs[bi].vu, bc = cs[bi].cl, bs = cs[bi].sm, bcc = cs[bi].cc;
             // then the block shapes of the bulk kernels under that schedule

@@ -1,5 +1,6 @@
 // Shared host-side helpers: thread-local error message and status plumbing.
 #pragma once
+#include <array>
 #include <cstddef>
 #include <string>
 #include <vector>
@@ -28,6 +29,9 @@ int group_create(rmt3d_scene *const *scenes, int n, scene_group **out);
 // a scene's multigrid schedule, as groups must share it: v_down, v_up,
 // smoother mode, cluster launch, cluster coarse sub-cycle's largest level
 void scene_schedule(rmt3d_scene *s, int out[5]);
+// first level of each solve's V-cycles (MAC, FEM) that its cluster launch
+// takes (-1: none)
+std::array<int, 2> scene_cluster_levels(const rmt3d_scene *s);
 int group_launch(scene_group *g, int nsteps);
 int group_finish(scene_group *g, int *status);
 // true once the group's launched steps have all run (group_finish then

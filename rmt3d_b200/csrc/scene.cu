@@ -2943,6 +2943,7 @@ void scene_schedule(rmt3d_scene *s, int out[5]) {
     out[3] = s->mac.use_cluster ? 1 : 0;
     out[4] = s->mac.cluster_coarse_pts;
 }
+std::array<int, 2> scene_cluster_levels(const rmt3d_scene *s) { return {s->mac.ccl, s->fem.ccl}; }
 }  // namespace rmt3d
 
 extern "C" int rmt3d_scene_set_coarse_cluster(rmt3d_scene *s, int pts) {

@@ -112,6 +112,43 @@ def test_autotune_choices_and_results(tmp_path):
         b.close()
 
 
+@pytest.mark.parametrize("n,precision,limit", [(24, R.FP64, 40000), (48, R.MIXED, R.COARSE_CLUSTER_ALL)])
+def test_autotune_keeps_a_new_scenes_cluster_launch(tmp_path, n, precision, limit):
+    """Where every candidate fails on the probe (here each step does: one
+    extrapolated layer is too few for the finite differences), a scene keeps
+    the cluster launch it was created with; the limit that hands over the same
+    levels (all that fit: at 48^3 mixed more than 40000 points) is reported."""
+    d = R.desc_from_cfg(scenes.write(str(tmp_path / "a.cfg"), scenes.cavity_sphere(n)))
+    d.precision, d.nlayers, d.num_iters = precision, 1, 0
+    b = R.Batch([d])
+    try:
+        b.prepare()
+        assert b.autotune(probe_steps=1) == {n ** 3: (2, 2, 0, 0, limit, 0)}
+    finally:
+        b.close()
+
+
+def test_cluster_launch_of_a_new_scene_asked_for_again(tmp_path):
+    """Naming a smoother drops a new scene's cluster launch; COARSE_CLUSTER_ALL
+    brings it back: the launches and the bits of a new scene."""
+    cfg = scenes.write(str(tmp_path / "c.cfg"), scenes.cavity(48))
+    got = []
+    for back in (False, True):
+        sc = R.Scene.from_cfg(cfg, precision=R.MIXED)
+        try:
+            if back:
+                sc.set_smoother(0)
+                sc.set_coarse_cluster(R.COARSE_CLUSTER_ALL)
+            sc.prepare()
+            assert sc.run(2) == R.NORMAL_EXIT
+            got.append((sc.launches(), [sc.field(f).copy() for f in ("u", "v", "w", "p")]))
+        finally:
+            sc.close()
+    assert got[0][0] == got[1][0]
+    for a, c in zip(got[0][1], got[1][1]):
+        assert np.array_equal(a, c)
+
+
 def test_footprint_is_what_a_scene_allocates(tmp_path):
     for d in _descs(tmp_path):
         for prec in (R.FP64, R.MIXED, R.MIXED_BULK32):
