@@ -6,6 +6,7 @@ import pytest
 
 import helpers as H
 import rmt3d_b200 as R
+from rmt3d_b200 import scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -20,6 +21,34 @@ def test_whole_cycle_bit_identical(tmp_path, name, precision):
     got, launches = [], []
     for pts in (None, 0):
         sc = R.Scene.from_cfg(cfg, precision=precision, var_den=int(fx.get("varden", 0)))
+        try:
+            if pts is not None:
+                sc.set_coarse_cluster(pts)
+            sc.prepare()
+            assert sc.run(3) == R.NORMAL_EXIT
+            got.append({f: sc.field(f).copy() for f in FIELDS})
+            launches.append(sc.launches())
+        finally:
+            sc.close()
+    for f in FIELDS:
+        assert np.array_equal(got[0][f], got[1][f]), f
+    assert launches[0] < launches[1]
+
+
+# the part starts below the finest level (64^3 from 33^3, 96^3 from 48^3 MAC
+# and 49^3 FEM in FP32), or is the whole cycle with three planes a CTA (48^3); in a
+# box periodic in z alone the sends wrap round the cluster
+@pytest.mark.parametrize("n,precision,var_den,periodic", [
+    (48, R.MIXED, 0, ""), (48, R.MIXED, 1, ""), (64, R.MIXED, 0, ""), (64, R.FP64, 1, ""), (96, R.MIXED, 0, ""),
+    (32, R.FP64, 0, "z"), (48, R.MIXED, 1, "z"), (64, R.MIXED, 0, "z"), (64, R.MIXED, 0, "xyz"), (48, R.MIXED, 1, "y")])
+def test_part_bit_identical(tmp_path, n, precision, var_den, periodic):
+    t = scenes.stretched_sphere(n) if periodic == "xyz" else scenes.cavity_sphere(n, rho=1.2 if var_den else 1.0)
+    t = t.replace("bc_yh 1 1 1 0 0 0", "bc_yh 1 1 1 0.5 0 0")
+    cfg = scenes.write(str(tmp_path / "s.cfg"),
+                       "".join(q + "\n" for q in t.splitlines() if not (q.startswith("bc_") and q[3] in periodic)))
+    got, launches = [], []
+    for pts in (None, 0):
+        sc = R.Scene.from_cfg(cfg, precision=precision, var_den=var_den)
         try:
             if pts is not None:
                 sc.set_coarse_cluster(pts)
