@@ -54,7 +54,7 @@ __device__ __forceinline__ void halo_arm(uint64_t *bar, unsigned bytes) {
 }
 // false if the phase did not complete within the limit (every send belongs to
 // a pass the sender has begun, so this does not happen; the bound keeps a
-// fault from turning into a hang)
+// fault from turning into a hang; a wait takes 4 us, so about 4 s)
 __device__ __forceinline__ bool halo_wait(uint64_t *bar, unsigned parity) {
     const unsigned b = (unsigned)__cvta_generic_to_shared(bar);
     for (int it = 0; it < (1 << 20); it++) {
@@ -67,6 +67,10 @@ __device__ __forceinline__ bool halo_wait(uint64_t *bar, unsigned parity) {
         if (ok) return true;
     }
     return false;
+}
+// about a millisecond, a thousand times what a send takes
+__device__ __forceinline__ void cl_linger() {
+    for (int it = 0; it < 16; it++) __nanosleep(64000);
 }
 
 }  // namespace rmt3d

@@ -886,7 +886,7 @@ double mg_solver::run(cudaStream_t st) {
         if (launches) *launches += outside_kernels + (h_ctl->cycles_total - before) * body_kernels;
     }
     sync_host_mirror();
-    return h_ctl->res_out;
+    return h_ctl->nan ? NAN : h_ctl->res_out;
 }
 
 }  // namespace rmt3d

@@ -283,6 +283,7 @@ pmg_args level_args(const mg_solver &m) {
     A.dense = m.dense;
     A.v_up = m.v_up;
     A.v_down = m.v_down;
+    A.gave_up = &m.ctl->gave_up;
     return A;
 }
 

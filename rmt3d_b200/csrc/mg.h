@@ -62,8 +62,9 @@ struct mg_ctl {
     int count;         // cycles of the current solve
     int last_cycles;   // cycles of the last finished solve
     int active;        // the current solve continues
-    int nan;           // the last solve ended with a NaN residual
+    int nan;           // the last solve ended with a NaN residual, or a wait in it gave up
     int need_res;      // the next iteration ends at a point where the control reads the residual
+    int gave_up;       // a wait of the current solve's cluster launches gave up (mg_slab.cuh)
     long long cycles_total;
     double V_avg, V_var;
     double prev, res_out;  // previous / reported max-norm residual

@@ -520,6 +520,7 @@ __device__ __forceinline__ void mg_begin_state(mg_ctl *c, unsigned long long *mx
     c->extra = 0;
     c->it = 0;
     c->count = 0;
+    c->gave_up = 0;
     c->active = 1;
     c->need_res = c->todo == 1;
     mx[0] = 0;
@@ -583,7 +584,7 @@ __device__ __forceinline__ bool mg_ctl_step(mg_ctl *c, unsigned long long *mx, d
         c->V_var = (1 - alpha) * (c->V_var + alpha * dV * dV);
         c->last_cycles = c->count;
         c->active = 0;
-        c->nan = (c->res_out != c->res_out);
+        c->nan = c->res_out != c->res_out || c->gave_up;
     }
     // the residual is read only where a phase ends (and every cycle of the
     // stagnation loop): the next iteration computes it only then

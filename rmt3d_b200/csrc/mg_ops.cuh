@@ -271,6 +271,7 @@ struct pmg_args {
     pmg_level lv[kMaxLev];
     const double *dense;  // inverse of the coarsest operator, or null
     int v_up, v_down;
+    int *gave_up;  // the solve's mg_ctl::gave_up (the shared-memory V-cycle sets it)
 };
 
 // the columns (or rows) of one parity: their number, the number off the rim

@@ -61,7 +61,7 @@ struct slab_ctx {
     T *sm;             // this CTA's shared memory
     int rank, tid;
     uint64_t *bar;     // two mbarriers for the neighbours' values, used in turn
-    int *failed;       // a wait on one of them gave up
+    int *failed;       // a wait on one of them gave up (set by the thread that waits)
 };
 
 // offset of column i within a row: columns -1..n0 as i+1, even ones first
@@ -433,10 +433,13 @@ __device__ __forceinline__ void colour_pass(const slab_ctx<T> &C, const slab_pas
 // planes, at the cluster barrier).  A neighbour may run one pass ahead -- it
 // then has all this CTA's rim values, so the ghost plane it writes has been
 // read -- hence two mbarriers in turn.  `use` counts the passes of the whole
-// cluster; CTAs without planes take part with nothing to wait for.
+// cluster; CTAs without planes take part with nothing to wait for.  After a wait
+// that gave up a CTA sends its values on, so that no other waits for it, but
+// neither waits nor arms: the phase it gave up on may still be open, and a
+// second arrival in it is not allowed (waits: this thread is the one that does).
 template <typename T, int KIND, bool VD>
 __device__ __forceinline__ void smooth_level(const slab_ctx<T> &C, const slab_view<T> &V,
-                                             int sweeps, const slab_pass *P, int &use) {
+                                             int sweeps, const slab_pass *P, int &use, bool &waits) {
     constexpr int nc = KIND == 1 ? 4 : 2;
     for (int s = 0; s < sweeps * nc; s++) {
         const int colour = s % nc;
@@ -445,9 +448,12 @@ __device__ __forceinline__ void smooth_level(const slab_ctx<T> &C, const slab_vi
             // one thread of the last warp, which has the fewest points, waits for
             // the neighbours; the block barrier hands on what it saw (every
             // warp polling cost a quarter of a pass's issue slots)
-            if (C.tid == kSlabThreads - 1) halo_arm(bar, P[colour].bytes);
+            if (waits) halo_arm(bar, P[colour].bytes);
             colour_pass<T, KIND, VD, 0>(C, P[colour], V, colour, use);
-            if (C.tid == kSlabThreads - 1 && *C.failed == 0 && !halo_wait(bar, (use >> 1) & 1)) *C.failed = 1;
+            if (waits && !halo_wait(bar, (use >> 1) & 1)) {
+                *C.failed = 1;
+                waits = false;
+            }
             __syncthreads();
             use++;
         } else {
@@ -662,6 +668,7 @@ __device__ __forceinline__ void slab_cycle(const pmg_args &A, const slab_args &S
     C.failed = reinterpret_cast<int *>(raw + S.bar_off + 2 * sizeof(uint64_t));
     const int nl = S.nlev;
     int use = 0;
+    bool waits = C.tid == kSlabThreads - 1;
     if (C.tid == 0) {
         halo_init(C.bar);
         halo_init(C.bar + 1);
@@ -724,7 +731,7 @@ __device__ __forceinline__ void slab_cycle(const pmg_args &A, const slab_args &S
     for (int l = 0; l < nl - 1; l++) {
         const slab_level &L = S.lv[l];
         const slab_view<T> V = view_of(C, L);
-        smooth_level<T, KIND, VD>(C, V, A.v_down, pass + 4 * l, use);
+        smooth_level<T, KIND, VD>(C, V, A.v_down, pass + 4 * l, use, waits);
         for (int c = 0; c < nc; c++) colour_pass<T, KIND, VD, 1>(C, pass[4 * l + c], V, c, -1);
         cl_barrier();
         restrict_level<T, KIND>(C, S, L, S.lv[l + 1], l + 1 == nl - 1);
@@ -737,7 +744,7 @@ __device__ __forceinline__ void slab_cycle(const pmg_args &A, const slab_args &S
         const slab_view<T> V = view_of(C, L);
         prolong_level<T, KIND>(C, L, S.lv[l + 1], V);
         cl_barrier();
-        smooth_level<T, KIND, VD>(C, V, A.v_up, pass + 4 * l, use);
+        smooth_level<T, KIND, VD>(C, V, A.v_up, pass + 4 * l, use, waits);
         cl_barrier();  // the next finer level reads x across slabs; no CTA leaves with sends under way
     }
     {
@@ -750,9 +757,14 @@ __device__ __forceinline__ void slab_cycle(const pmg_args &A, const slab_args &S
             const int row = fdiv(t, L.inv_n0), i = t - row * L.n0;
             const int kl = fdiv(row, L.inv_n1), j = row - kl * L.n1;
             const T v = C.sm[L.ox + (kl + 1) * L.PX + (j + 1) * L.RS + col(L, i)];
-            // a wait that gave up shows as NaN, which the solve's control reports
             gx[g0 + t] = *C.failed ? (T)NAN : v;
         }
+    }
+    // a wait that gave up: the solve's control reports it, and this CTA stays
+    // until what is still under way to its shared memory has arrived
+    if (*C.failed) {
+        if (C.tid == 0) *A.gave_up = 1;
+        cl_linger();
     }
 }
 

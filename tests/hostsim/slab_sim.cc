@@ -4,7 +4,10 @@
 // its term-by-term form (ref_ops.inc).  Built with the
 // address sanitizer, every CTA's shared memory a heap block of its own size,
 // so an index outside it ends the run.
-//   slab_sim kind(0 MAC, 1 FEM) vd f64 n0 n1 n2 p0 p1 p2 csize v_down v_up l0 seed
+//   slab_sim kind(0 MAC, 1 FEM) vd f64 n0 n1 n2 p0 p1 p2 csize v_down v_up l0 seed [drop]
+// With `drop`, that value of those sent to CTA 1 is lost, so its wait gives
+// up: every thread still ends, no mbarrier is armed twice in a phase, CTA 1's planes
+// come out NaN and the solve's control, given that residual, reports NaN.
 #include <atomic>
 #include <barrier>
 #include <chrono>
@@ -12,6 +15,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <random>
 #include <thread>
 
@@ -29,10 +33,10 @@ std::vector<cta_state> g_cta;
 std::barrier<> *g_all = nullptr;
 thread_local int t_rank = 0;
 struct dim {
-    int x;
+    int x, y, z;
 };
 }  // namespace
-thread_local dim threadIdx{0}, blockDim{1};
+thread_local dim threadIdx{0, 0, 0}, blockDim{1, 1, 1};
 inline void __syncthreads() {
     if (!g_cta.empty()) g_cta[t_rank].bar->arrive_and_wait();
 }
@@ -44,6 +48,23 @@ inline double __shfl_xor_sync(unsigned, double v, int o) {
     const double r = c.lane[threadIdx.x ^ o];
     c.bar->arrive_and_wait();
     return r;
+}
+// for the control (mg_body.cuh)
+inline unsigned long long __shfl_xor_sync(unsigned, unsigned long long v, int) { return v; }
+inline long long __double_as_longlong(double v) {
+    long long b;
+    memcpy(&b, &v, 8);
+    return b;
+}
+inline double __longlong_as_double(long long b) {
+    double v;
+    memcpy(&v, &b, 8);
+    return v;
+}
+inline unsigned long long atomicMax(unsigned long long *p, unsigned long long v) {
+    const unsigned long long o = *p;
+    if (v > o) *p = v;
+    return o;
 }
 inline unsigned __umulhi(unsigned a, unsigned b) { return (unsigned)(((uint64_t)a * b) >> 32); }
 
@@ -74,8 +95,12 @@ inline void sim_step(sim_bar *b, int d) {
         b->phase.fetch_add(1);
     }
 }
+int g_drop = -1;  // which value sent to CTA 1 is lost (-1: none)
+std::atomic<int> g_sent{0}, g_rearmed{0};
 template <typename T>
 void cl_send(cl_addr a, T v, cl_addr bar) {
+    const bool to1 = g_drop >= 0 && (unsigned char *)bar >= g_cta[1].smem && (unsigned char *)bar < g_cta[1].smem + g_cta[1].bytes;
+    if (to1 && g_sent.fetch_add(1) == g_drop) return;
     *(T *)a = v;
     sim_step((sim_bar *)bar, -(int)sizeof(T));
 }
@@ -84,17 +109,25 @@ inline void halo_init(uint64_t *b) {
     ((sim_bar *)b)->phase = 0;
 }
 inline void halo_init_fence() {}
-inline void halo_arm(uint64_t *b, unsigned bytes) { sim_step((sim_bar *)b, (int)bytes - kUnarmed); }
+inline void halo_arm(uint64_t *b, unsigned bytes) {
+    if (((sim_bar *)b)->due < kUnarmed / 2) g_rearmed++;  // the phase's one arrival has come already
+    sim_step((sim_bar *)b, (int)bytes - kUnarmed);
+}
 inline bool halo_wait(uint64_t *b, unsigned parity) {
-    for (int it = 0; it < 4000000; it++) {
+    for (int it = 0; it < (g_drop < 0 ? 4000000 : 8000); it++) {
         if ((((sim_bar *)b)->phase & 1) != (int)parity) return true;
         std::this_thread::sleep_for(std::chrono::microseconds(20));
     }
     return false;
 }
+inline void cl_linger() {}
 int fail(int code, const std::string &) { return code; }
 }  // namespace rmt3d
 #include "mg_slab.cuh"
+
+using std::max;
+using std::min;
+#include "mg_body.cuh"
 
 namespace rmt3d {
 #include "ref_ops.inc"
@@ -168,6 +201,8 @@ static int run(const std::vector<mg_level> &lv, int csize, int vdn, int vup, int
     std::vector<double> B(np * np);
     for (auto &v : B) v = U(rng) / np;
     A.dense = B.data();
+    int gave_up = 0;
+    A.gave_up = &gave_up;
     for (int l = 0; l < A.nlev; l++) {
         for (int d = 0; d < 3; d++) A.lv[l].n[d] = lv[l].n[d], A.lv[l].prd[d] = lv[l].prd[d];
         set_level_ptrs<T>(A.lv[l], x[l].data(), r[l].data(), s[l].data());
@@ -189,6 +224,7 @@ static int run(const std::vector<mg_level> &lv, int csize, int vdn, int vup, int
     g_cta.assign(csize, cta_state());
     for (auto &c : g_cta) {
         c.smem = (unsigned char *)aligned_alloc(16, (bytes + 15) & ~(size_t)15);
+        c.bytes = bytes;
         memset(c.smem, 0xff, bytes);  // NaN: reads of what was never written show
         c.bar = new std::barrier<>(RMT3D_SLAB_THREADS);
     }
@@ -208,6 +244,23 @@ static int run(const std::vector<mg_level> &lv, int csize, int vdn, int vup, int
         delete c.bar;
     }
     g_cta.clear();
+    if (g_drop >= 0) {
+        const slab_level &L = S.lv[0];
+        const size_t pl = (size_t)L.n0 * L.n1;
+        size_t numbers = 0;
+        for (size_t q = pl * L.q; q < pl * std::min(2 * L.q, L.n2); q++) numbers += got[q] == got[q];
+        // the control at the end of the solve (its last cycles read no residual)
+        mg_ctl c;
+        memset(&c, 0, sizeof(c));
+        unsigned long long mx[2] = {0, 0};
+        mg_begin_state(&c, mx);
+        c.phase = 2;
+        c.todo = 1;
+        c.gave_up = gave_up;
+        const bool done = mg_ctl_step(&c, mx, 1, 0, 0);
+        printf("given up %d, armed twice %d, numbers in CTA 1's planes %zu, nan %d\n", gave_up, g_rearmed.load(), numbers, c.nan);
+        return gave_up && !g_rearmed && !numbers && done && c.nan ? 0 : 6;
+    }
     x[l0] = x0;
     // the per-phase cycle, one thread; the dense solve in 32 lanes' order
     threadIdx.x = 0;
@@ -243,14 +296,16 @@ static int run(const std::vector<mg_level> &lv, int csize, int vdn, int vup, int
             if (!bad) printf("first difference at %zu: %.17g %.17g\n", q, (double)got[q], (double)x[l0][q]);
             bad++;
         }
+    if (gave_up || g_rearmed) return 7;
     printf("levels %d points %zu bytes/CTA %zu different %zu\n", A.nlev - l0, got.size(), bytes, bad);
     return bad ? 1 : 0;
 }
 
 int main(int argc, char **argv) {
-    if (argc != 15) return 3;
+    if (argc != 15 && argc != 16) return 3;
     int a[14];
     for (int i = 0; i < 14; i++) a[i] = atoi(argv[i + 1]);
+    if (argc == 16) g_drop = atoi(argv[15]);
     const int n[3] = {a[3], a[4], a[5]}, prd[3] = {a[6], a[7], a[8]};
     std::vector<mg_level> lv;
     if (plan(a[0], n, prd, lv)) return 4;

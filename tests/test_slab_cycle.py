@@ -46,3 +46,19 @@ def sim(tmp_path_factory):
 def test_slab_cycle_matches_phases(sim, args):
     r = subprocess.run([sim] + args.split() + ["7"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr[-2000:]
+
+
+# kind, density, type, points, periodic, CTAs, sweeps, first level; the value sent to
+# CTA 1 that is lost: of the first pass, and of the last (of the cycle's 2,000
+# or so), after which nothing waits
+@pytest.mark.parametrize("args,drop", [
+    ("1 0 1 17 17 17 0 0 0 5 2 2 0", 3),
+    ("0 1 0 16 16 16 0 0 0 4 1 2 0", 40),
+    ("1 1 0 17 17 16 0 0 1 4 2 1 0", 1700),
+])
+def test_wait_that_gives_up_is_reported(sim, args, drop):
+    """A neighbour's value that never arrives: the wait gives up, every thread
+    still reaches the end, no mbarrier gets a second arrival in a phase, the
+    waiting CTA's planes come out NaN and the solve's control reports it."""
+    r = subprocess.run([sim] + args.split() + ["7", str(drop)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr[-2000:]
