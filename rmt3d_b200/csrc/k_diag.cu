@@ -11,8 +11,7 @@ namespace rmt3d {
 // that finishes last) the blocks in index order.  Bit c of max_mask makes
 // value c a maximum instead of a sum.  out holds NV totals followed by NV
 // partials per block; *ticket returns to 0.  blockDim.x is a multiple of 32,
-// gridDim.x at most kRedBlocks.
-constexpr int kRedBlocks = 148;
+// gridDim.x at most kMeanBlocks.
 template <int NV>
 __device__ void fixed_order_reduce(double (&v)[NV], unsigned max_mask, double *out, unsigned *ticket) {
     __shared__ double sh[NV][32];
@@ -42,7 +41,7 @@ __device__ void fixed_order_reduce(double (&v)[NV], unsigned max_mask, double *o
     // the whole block fetches the partials, one thread a value adds them in
     // block order (fetching them one by one as well was a chain of 148 L2
     // latencies)
-    __shared__ double part[NV * kRedBlocks];
+    __shared__ double part[NV * kMeanBlocks];
     __threadfence();
     for (int t = threadIdx.x; t < NV * (int)gridDim.x; t += blockDim.x) part[t] = __ldcg(out + NV + t);
     __syncthreads();

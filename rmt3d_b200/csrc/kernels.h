@@ -38,6 +38,10 @@ struct bc_faces {
     bc_face f[6];
 };
 
+// Blocks of a fixed-order reduction over the grid (the mean, the diagnostics):
+// its launches, the partials' scratch and the last block's shared copy of them.
+constexpr int kMeanBlocks = 148;
+
 // FEM element-integrated basis gradients (fluid_3d.cc:2506-2517)
 struct gradphi_t {
     double v[8][3];

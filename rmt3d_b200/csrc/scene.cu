@@ -964,7 +964,6 @@ static void ph_ustar(rmt3d_scene *s) {
 // and the last block to finish adds the partials in block order, so the
 // result does not depend on scheduling (scenes give the same answer alone
 // and when they share the device with others).
-constexpr int kMeanBlocks = 148;
 constexpr int kDiagVals = 8;
 
 __global__ void k_mean(const double *x, size_t n, double scale, double *out, unsigned *ticket) {
