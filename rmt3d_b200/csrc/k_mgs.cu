@@ -59,24 +59,21 @@ cudaError_t slab_go(const void *fn, void **args, int clusters, int csize, size_t
 }
 }  // namespace
 
-// the kernels' attributes, and whether a cluster of csize CTAs with the
-// largest shared memory fits this device (once per device)
-int slab_cluster_size() {
-    static std::mutex mu;
-    static int size[64];
-    static bool done[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done[dev]) return size[dev];
-    done[dev] = true;
-    size[dev] = 0;
+// the kernels' attributes, the largest cluster whose CTAs fit this device with
+// the largest shared memory (0: neither 16 nor 8), and how many such clusters
+// run at once (once per device)
+namespace {
+struct slab_device {
+    int size = 0, at_once = 0;
+};
+slab_device query_device() {
+    slab_device q;
     for (int m = 0; m < 16; m++) {
         const void *fn = slab_fn(m & 1, m & 2, m & 4, m & 8);
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
             cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmemMax) != cudaSuccess) {
             cudaGetLastError();
-            return 0;
+            return q;
         }
     }
     for (int c : {16, 8}) {
@@ -100,10 +97,36 @@ int slab_cluster_size() {
             }
             least = std::min(least, n);
         }
-        if (least >= 1) return size[dev] = c;
+        if (least >= 1) {
+            q.size = c;
+            q.at_once = least;
+            break;
+        }
     }
-    return 0;
+    return q;
 }
+slab_device this_device() {
+    static std::mutex mu;
+    static slab_device known[64];
+    static bool done[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return slab_device();
+    std::lock_guard<std::mutex> lk(mu);
+    if (!done[dev]) known[dev] = query_device();
+    done[dev] = true;
+    return known[dev];
+}
+}  // namespace
+
+int slab_cluster_size() { return this_device().size; }
+
+// A group's clusters, one a scene, run in waves of as many as fit the device (7
+// of 16 CTAs on a B200), while its per-phase launches fill the device with all
+// scenes' points.  Against those, step time of groups of 12^3 to 96^3 scenes,
+// both densities, FP64 and mixed: one wave 1.03 to 1.5 times as fast, two
+// waves (8 to 14 scenes) 0.84 to 1.11, three (15) 0.73 to 0.99, five (32) 0.61
+// to 0.91.
+bool slab_pays(int scenes) { return scenes <= 2 * this_device().at_once; }
 
 bool slab_fits(const mg_solver &m, int l0) {
     const size_t b = slab_layout(m.lv, l0, m.slab_csize, !m.mixed, m.vd, false, nullptr);

@@ -2943,6 +2943,7 @@ void scene_schedule(rmt3d_scene *s, int out[5]) {
     out[4] = s->mac.cluster_coarse_pts;
 }
 std::array<int, 2> scene_cluster_levels(const rmt3d_scene *s) { return {s->mac.ccl, s->fem.ccl}; }
+bool group_cluster_pays(int scenes) { return slab_pays(scenes); }
 }  // namespace rmt3d
 
 extern "C" int rmt3d_scene_set_coarse_cluster(rmt3d_scene *s, int pts) {
@@ -2950,6 +2951,7 @@ extern "C" int rmt3d_scene_set_coarse_cluster(rmt3d_scene *s, int pts) {
     if (pts < 0) return fail(RMT3D_ERR_INVALID, "negative level size");
     if (pts > 0 && (!s->mac.slab_csize || !s->fem.slab_csize))
         return fail(RMT3D_ERR_UNSUPPORTED, "thread-block clusters of 8 or more CTAs are not available");
+    if (pts == RMT3D_COARSE_CLUSTER_ALL) pts = kSlabAuto;
     s->mac.set_cluster_coarse(pts);
     s->fem.set_cluster_coarse(pts);
     mark_dirty(s);
