@@ -346,9 +346,9 @@ int rmt3d_write_slice(rmt3d_scene *s, int type, int dim, int point, int obj_id, 
  * most 274,625 FEM nodes (65^3, a 64^3 box with walls); larger grids return
  * RMT3D_ERR_TOO_LARGE.  No cudaMalloc/cudaFree or allocating library call is
  * made.  Each call looks the array's device address up on the current device
- * (cudaGetSymbolAddress) and waits for `stream` before returning the value: the call is synchronous and
- * must not be issued on a stream that is capturing.  Every call shares the
- * array: calls that overlap on the GPU race.
+ * (cudaGetSymbolAddress) and waits for `stream` before returning the value:
+ * the call is synchronous and must not be issued on a stream that is
+ * capturing.  Every call shares the array: calls that overlap on the GPU race.
  *   dvel[3]: du, dv, dw over the ghosted box (sys_size+4 per axis), with the
  *   two ghost layers filled as the step leaves them (on a periodic axis they
  *   hold the periodic images, which the FEM right-hand side reads);

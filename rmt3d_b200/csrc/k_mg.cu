@@ -16,7 +16,8 @@
 //  * Coarsest level: a dense inverse of A + (alpha/n) 1 1^T, precomputed on the
 //    host; for the singular Neumann/periodic operators (null space = the
 //    constants) it returns the solution orthogonal to the constants.
-// Residual max norms are reduced with warp shuffles and one atomic per warp.
+// Residual max norms are reduced with warp shuffles and at most one atomic per
+// block.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

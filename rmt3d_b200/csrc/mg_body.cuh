@@ -267,8 +267,9 @@ __device__ __forceinline__ void body_resid_to_f32(lvl_dev L, const double *__res
 }
 
 // the block's maximum of b into *mx: one atomic per block, none where the
-// maximum so far already covers it (an atomic per warp made the 192^3 MAC norm
-// 63 us; now 31).  Every thread of the block calls it.
+// maximum so far already covers it.  Every thread of the block calls it.  B200,
+// 192^3, by ncu: the right-hand side's norm 16 us, with an atomic per warp 19;
+// the marching residual norms take 41 (MAC) and 75 us (FEM) either way.
 __device__ __forceinline__ void block_max_into(unsigned long long b, unsigned long long *mx) {
     __shared__ unsigned long long wmax[32];
     for (int o = 16; o > 0; o >>= 1) {

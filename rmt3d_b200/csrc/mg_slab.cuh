@@ -6,19 +6,21 @@
 // variable density of 1/rho; the residual of the level being restricted has
 // one buffer for all levels.  A colour pass reads shared memory only, writes
 // the new values home and, for the first and last plane of the slab, into
-// the neighbours' ghost planes (distributed shared memory), and ends with the
-// hardware cluster barrier.  Ghost columns and rows hold the periodic images,
-// or zero beyond a wall; adding a zero term leaves every sum's bits alone, so
-// boundary and interior points run the same loads and the boundary rules
-// reduce to coefficients.  Every point's sum has the order of the per-phase
-// kernels (mg_ops.cuh): the same bits as one launch per phase.
+// the neighbours' ghost planes (distributed shared memory).  It ends when the
+// neighbours' values of the pass have arrived, counted on an mbarrier, or, with
+// periodic images within the planes, at the hardware cluster barrier.  Ghost
+// columns and rows hold the periodic images, or zero beyond a wall; adding a
+// zero term leaves every sum's bits alone, so boundary and interior points run
+// the same loads and the boundary rules reduce to coefficients.  Every point's
+// sum has the order of the per-phase kernels (mg_ops.cuh): the same bits as one
+// launch per phase.
 //
 // What bounds it: these levels have 10^2..10^5 points, and a phase issued as
 // its own launch costs the launch and one or two dependent L2 latencies
 // (2.5-4 us) whatever its size.  Here a phase costs its points' instructions
 // on 16 SMs and a hand-over: 0.45-1.2 us a colour pass, of which 0.15-0.3 us
 // is the wait for the neighbours (a full cluster barrier measured 0.3 us).
-// Measured on a B200: the V(2,1) part from 33^3 down, FP32, 49 us against
+// Measured on a B200: the V(2,1) part from 33^3 down, FP32, 47 us against
 // about 120 us for its 34 launches, MAC from 32^3 27 against 65 us; a
 // 16^3 FP64 cavity step 761 -> 430 us, a 64^3 mixed step with a sphere
 // 1.41 -> 1.21 ms.
@@ -43,9 +45,9 @@
 
 namespace rmt3d {
 
-// Threads per CTA.  512 measured fastest: the V(2,1) part of a 33^3 FP32
-// hierarchy takes 49 us, against 56 us with 256 and 53 us with 1024 threads
-// (whose 64 registers spill).
+// Threads per CTA.  512 measured fastest, in an earlier form whose warps all
+// polled for the neighbours: the V(2,1) part of a 33^3 FP32 hierarchy took 49 us,
+// against 56 us with 256 and 53 us with 1024 threads (whose 64 registers spill).
 #ifndef RMT3D_SLAB_THREADS
 #define RMT3D_SLAB_THREADS 512
 #endif
