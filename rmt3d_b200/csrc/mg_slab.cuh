@@ -438,10 +438,10 @@ __device__ __forceinline__ void colour_pass(const slab_ctx<T> &C, const slab_pas
 // cluster; CTAs without planes take part with nothing to wait for.  After a wait
 // that gave up a CTA sends its values on, so that no other waits for it, but
 // neither waits nor arms: the phase it gave up on may still be open, and a
-// second arrival in it is not allowed (waits: this thread is the one that does).
+// second arrival in it is not allowed.
 template <typename T, int KIND, bool VD>
 __device__ __forceinline__ void smooth_level(const slab_ctx<T> &C, const slab_view<T> &V,
-                                             int sweeps, const slab_pass *P, int &use, bool &waits) {
+                                             int sweeps, const slab_pass *P, int &use) {
     constexpr int nc = KIND == 1 ? 4 : 2;
     for (int s = 0; s < sweeps * nc; s++) {
         const int colour = s % nc;
@@ -449,12 +449,13 @@ __device__ __forceinline__ void smooth_level(const slab_ctx<T> &C, const slab_vi
             uint64_t *bar = C.bar + (use & 1);
             // one thread of the last warp, which has the fewest points, waits for
             // the neighbours; the block barrier hands on what it saw (every
-            // warp polling cost a quarter of a pass's issue slots)
-            if (waits) halo_arm(bar, P[colour].bytes);
+            // warp polling cost a quarter of a pass's issue slots).  It arms here
+            // too: values that came before lower the phase's byte count below zero
+            // and cannot end it, as its one arrival is still due.
             colour_pass<T, KIND, VD, 0>(C, P[colour], V, colour, use);
-            if (waits && !halo_wait(bar, (use >> 1) & 1)) {
-                *C.failed = 1;
-                waits = false;
+            if (C.tid == kSlabThreads - 1 && *C.failed == 0) {
+                halo_arm(bar, P[colour].bytes);
+                if (!halo_wait(bar, (use >> 1) & 1)) *C.failed = 1;
             }
             __syncthreads();
             use++;
@@ -670,7 +671,6 @@ __device__ __forceinline__ void slab_cycle(const pmg_args &A, const slab_args &S
     C.failed = reinterpret_cast<int *>(raw + S.bar_off + 2 * sizeof(uint64_t));
     const int nl = S.nlev;
     int use = 0;
-    bool waits = C.tid == kSlabThreads - 1;
     if (C.tid == 0) {
         halo_init(C.bar);
         halo_init(C.bar + 1);
@@ -733,7 +733,7 @@ __device__ __forceinline__ void slab_cycle(const pmg_args &A, const slab_args &S
     for (int l = 0; l < nl - 1; l++) {
         const slab_level &L = S.lv[l];
         const slab_view<T> V = view_of(C, L);
-        smooth_level<T, KIND, VD>(C, V, A.v_down, pass + 4 * l, use, waits);
+        smooth_level<T, KIND, VD>(C, V, A.v_down, pass + 4 * l, use);
         for (int c = 0; c < nc; c++) colour_pass<T, KIND, VD, 1>(C, pass[4 * l + c], V, c, -1);
         cl_barrier();
         restrict_level<T, KIND>(C, S, L, S.lv[l + 1], l + 1 == nl - 1);
@@ -746,7 +746,7 @@ __device__ __forceinline__ void slab_cycle(const pmg_args &A, const slab_args &S
         const slab_view<T> V = view_of(C, L);
         prolong_level<T, KIND>(C, L, S.lv[l + 1], V);
         cl_barrier();
-        smooth_level<T, KIND, VD>(C, V, A.v_up, pass + 4 * l, use, waits);
+        smooth_level<T, KIND, VD>(C, V, A.v_up, pass + 4 * l, use);
         cl_barrier();  // the next finer level reads x across slabs; no CTA leaves with sends under way
     }
     {
