@@ -68,7 +68,7 @@ def test_part_bit_identical(tmp_path, n, precision, var_den, periodic):
 def test_large_group_runs_per_phase(tmp_path):
     """A group of more scenes than their clusters pay for runs its multigrid
     phases as launches over all scenes: as fast as when asked to (32 clusters
-    took 1.5 times as long on this box), with the same bits."""
+    took 1.5 times as long on a B200), with the same bits."""
     text = "".join(q + "\n" for q in scenes.cavity(12).splitlines() if not q.startswith("bc_"))
     d = R.desc_from_cfg(scenes.write(str(tmp_path / "p.cfg"), text))
     best, got = [], []
