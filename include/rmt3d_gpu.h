@@ -377,10 +377,10 @@ int rmt3d_scene_set_smoother(rmt3d_scene *s, int mode);
  * as many levels as fit, until this call, rmt3d_scene_set_smoother (either
  * mode) or a one-block coarse sub-cycle (rmt3d_scene_set_schedule) chooses
  * otherwise; RMT3D_COARSE_CLUSTER_ALL, a limit no level exceeds, is a new
- * scene's choice again.  In a group, whose scenes run one cluster each, that
- * choice takes the launch while the clusters run in at most two waves (14
- * scenes on a B200); another limit takes it in any group.  No counterpart in
- * the reference. */
+ * scene's choice again.  A group, whose scenes run one cluster each, takes the
+ * launch while the clusters run in at most two waves (14 scenes on a B200) and
+ * runs per-phase launches over all scenes beyond.  No counterpart in the
+ * reference. */
 #define RMT3D_COARSE_CLUSTER_ALL 2147483647
 int rmt3d_scene_set_coarse_cluster(rmt3d_scene *s, int pts);
 

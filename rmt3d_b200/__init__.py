@@ -273,8 +273,9 @@ class Scene:
     def set_coarse_cluster(self, pts):
         """Run the V-cycles' levels of at most `pts` points that fit a
         thread-block cluster's shared memory as one launch per cycle; 0:
-        per-phase launches; COARSE_CLUSTER_ALL: a new scene's choice, every
-        level that fits, except in groups of many scenes (the same bits)."""
+        per-phase launches; COARSE_CLUSTER_ALL: every level that fits, as a
+        new scene has it.  Groups of many scenes run per-phase launches (the
+        same bits)."""
         _lib.check(lib().rmt3d_scene_set_coarse_cluster(self._h, int(pts)))
 
     def set_block_shape(self, shape):

@@ -260,7 +260,7 @@ extern "C" int rmt3d_batch_scene(rmt3d_batch *b, int i, rmt3d_scene **out) {
 // launch per colour pass, or one per whole sweep on shared-memory tiles) and
 // the levels (none, up to 5000 or 40000 points, or every one that fits, as a
 // new scene has it) whose part of each V-cycle runs as one cluster launch (for
-// kinds whose scenes make a group that runs it unasked).
+// kinds whose scenes make a group that runs it).
 // Where every candidate fails on the probe, a new scene's schedule stays.
 // With the fastest of those, the block shapes of the bulk stencil kernels are
 // timed the same way (rmt3d_scene_set_block_shape).  tuned_out (optional, 7
@@ -344,8 +344,8 @@ extern "C" int rmt3d_batch_autotune(rmt3d_batch *b, int probe_steps, int *tuned_
         int all = 0;  // a new scene's
         int kind = 0;
         for (auto &d : b->descs) kind += tune_key(d) == kv.first;
-        // the probe steps alone: it cannot tell what the launch costs a group
-        // of more scenes than their clusters pay for
+        // the probe steps alone, and would choose a launch that a group of so
+        // many scenes does not run
         const bool grouped = kind > 1 && !rmt3d::group_cluster_pays(kind);
         for (auto &ln : launch) {
             if (ln[2] > 0) {

@@ -32,7 +32,7 @@ void scene_schedule(rmt3d_scene *s, int out[5]);
 // first level of each solve's V-cycles (MAC, FEM) that its cluster launch
 // takes (-1: none)
 std::array<int, 2> scene_cluster_levels(const rmt3d_scene *s);
-// whether a group of so many new scenes runs that launch
+// whether a group of so many scenes runs that launch
 bool group_cluster_pays(int scenes);
 int group_launch(scene_group *g, int nsteps);
 int group_finish(scene_group *g, int *status);

@@ -227,7 +227,7 @@ int mg_group::setup(const std::vector<mg_solver *> &solvers, cudaStream_t st) {
             for (int d = 0; d < 3; d++) same = same && m->lv[l].n[d] == lv[l].n[d] && m->lv[l].prd[d] == lv[l].prd[d];
         if (!same) return fail(RMT3D_ERR_INVALID, "scenes of a multigrid group must match in size, form and schedule");
     }
-    if (s0.cluster_coarse_pts == kSlabAuto && !slab_pays(B)) ccl = -1;
+    if (!slab_pays(B)) ccl = -1;
     // one device block: per level 8 pointer tables of B entries, then the
     // control pointers, the residual slots' pointers and part/run flags
     const size_t L = lv.size();

@@ -131,7 +131,7 @@ class mg_solver {
     int ccl = -1;
     int slab_csize = 0;  // CTAs of that cluster (0: not available)
     // largest level handed to that launch: 0 none, kSlabAuto (a new scene)
-    // every level that fits, alone or in a group that slab_pays for
+    // every level that fits; in a group while slab_pays for it
     int cluster_coarse_pts = kSlabAuto;
     int set_cluster_coarse(int pts);
     // whether level l starts that launch (the launch profiler times the
@@ -180,7 +180,7 @@ class mg_solver {
 // cluster each)
 class mg_group;
 int slab_cluster_size();
-bool slab_pays(int scenes);  // whether a group of so many takes it unasked
+bool slab_pays(int scenes);  // whether a group of so many takes it
 bool slab_fits(const mg_solver &m, int l0);
 cudaError_t slab_cycle_launch(const mg_solver &m, int l0, bool f32, cudaStream_t st);
 cudaError_t slab_cycle_launch_b(const mg_group &g, int l0, bool f32, cudaStream_t st);

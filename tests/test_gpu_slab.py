@@ -67,12 +67,13 @@ def test_part_bit_identical(tmp_path, n, precision, var_den, periodic):
 
 def test_large_group_runs_per_phase(tmp_path):
     """A group of more scenes than their clusters pay for runs its multigrid
-    phases as launches over all scenes: as fast as when asked to (32 clusters
-    took 1.5 times as long on a B200), with the same bits."""
+    phases as launches over all scenes, new scenes and scenes with a limit
+    alike: as fast as when asked to (32 clusters took 1.5 times as long on a
+    B200), with the same bits."""
     text = "".join(q + "\n" for q in scenes.cavity(12).splitlines() if not q.startswith("bc_"))
     d = R.desc_from_cfg(scenes.write(str(tmp_path / "p.cfg"), text))
     best, got = [], []
-    for pts in (None, 0):
+    for pts in (None, 40000, 0):
         b = R.Batch([d] * 32)
         try:
             if pts is not None:
@@ -89,6 +90,6 @@ def test_large_group_runs_per_phase(tmp_path):
             got.append([b.field(31, f) for f in FIELDS])
         finally:
             b.close()
-    for f, a, c in zip(FIELDS, *got):
-        assert np.array_equal(a, c), f
-    assert best[0] < 1.25 * best[1]
+    for f, a, c, e in zip(FIELDS, *got):
+        assert np.array_equal(a, e) and np.array_equal(c, e), f
+    assert best[0] < 1.25 * best[2] and best[1] < 1.25 * best[2]
